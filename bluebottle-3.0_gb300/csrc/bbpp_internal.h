@@ -19,12 +19,13 @@ struct GraphKey {
   double bscale = 1.0;
   const void *xhi = nullptr, *rhs64 = nullptr;
   const void *r1 = nullptr, *Ap1 = nullptr;  // fused iterations: the second r and Ap buffers
+  bool persist = false;  // resident iterations
   cudaStream_t stream = nullptr;
   bool operator==(const GraphKey &o) const {
     return mask == o.mask && rhs == o.rhs && x == o.x && r == o.r && p0 == o.p0 && p1 == o.p1 && Ap == o.Ap &&
            st == o.st && len == o.len && replace_every == o.replace_every && elem == o.elem && rr == o.rr &&
            bscale == o.bscale && xhi == o.xhi && rhs64 == o.rhs64 && r1 == o.r1 && Ap1 == o.Ap1 &&
-           stream == o.stream;
+           stream == o.stream && persist == o.persist;
   }
 };
 
@@ -51,6 +52,7 @@ struct IrBuffers;   // FP32 inner-sweep workspace (bbpp_ir.cu)
 struct NetWork;     // learned-guess workspace (bbpp_net.cu)
 
 struct bbpp_tma_state;
+struct bbpp_persist_state;
 void *bbpp_tensor_map_encoder();  // cuTensorMapEncodeTiled, or null
 bool bbpp_tma_chunks(const bbpp_ctx *ctx, int *kz, int *nzc);  // z chunking of the TMA search kernel
 
@@ -89,6 +91,7 @@ struct bbpp_ctx {
   IrBuffers *ir = nullptr;
   NetWork *net = nullptr;
   bbpp_tma_state *tma = nullptr;  // launch shape and tensor maps of the TMA search kernel
+  bbpp_persist_state *persist = nullptr;  // boxes of the resident iteration (small grids)
   bool pdl = false;               // iteration kernels launch with a programmatic dependency
   bool rev_update = true;         // the update kernel walks the search kernel's planes in reverse
   bool l2hint = true;             // FP32 iteration: mask evict_last in L2, p / Ap / x evict_first
@@ -196,6 +199,15 @@ bool bbpp_tma_fused(bbpp_ctx *ctx, const uint8_t *mask, const float *rin, const 
 bool bbpp_tma_search(bbpp_ctx *ctx, const uint8_t *mask, const float *r, const float *pold, float *pnew, float *Ap,
                      float *x, bbpp::DevState *st);
 int bbpp_residual_async(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs, const double *x, double *r);
+
+// iterations up to the next checkpoint in one resident kernel (bbpp_persist.cu)
+void bbpp_persist_init(bbpp_ctx *ctx);
+void bbpp_persist_free(bbpp_ctx *ctx);
+bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem);
+int bbpp_persist_begin(bbpp_ctx *ctx);
+template <typename T>
+int bbpp_persist(bbpp_ctx *ctx, const uint8_t *mask, T *r, T *const p[2], T *Ap, T *x, bbpp::DevState *st,
+                 int replace_every);
 
 // learned initial guess (bbpp_net.cu)
 int bbpp_net_guess(bbpp_ctx *ctx, void *net, const uint8_t *mask, const double *rhs, const double *prev, double *x,

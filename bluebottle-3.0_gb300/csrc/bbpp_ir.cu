@@ -88,7 +88,7 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   bbpp_set_reliable(x, rhs);
   float *const p[2] = {b->p[0], b->p[1]};
   int it = 0;
-  bool fused = ctx->fused && bbpp_tma_fused_ok(ctx);
+  bool fused = ctx->fused && bbpp_tma_fused_ok(ctx) && !bbpp_persist_ok(ctx, 4);
   if (fused && !b->rd2) {
     CK(cudaMalloc(&b->rd2, sizeof(float) * n));
     CK(cudaMalloc(&b->Ap2, sizeof(float) * n));

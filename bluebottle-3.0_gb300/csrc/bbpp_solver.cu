@@ -251,6 +251,7 @@ extern "C" int bbpp_create(const bbpp_grid *g, bbpp_ctx **out) {
   ctx->sms = dev_sms();
   stencil_shape(ctx);
   bbpp_tma_init(ctx);
+  bbpp_persist_init(ctx);
   {
     // programmatic dependent launch of the iteration kernels: off unless
     // BBPP_PDL=1 (measured at 256^3: no gain, the kernels' own drain and fill
@@ -326,6 +327,7 @@ extern "C" int bbpp_destroy(bbpp_ctx *ctx) {
   bbpp_ir_free(ctx);
   bbpp_net_ctx_free(ctx);
   bbpp_tma_free(ctx);
+  bbpp_persist_free(ctx);
   if (ctx->st) cudaFree(ctx->st);
   if (ctx->trace) cudaFree(ctx->trace);
   if (ctx->partials) cudaFree(ctx->partials);
@@ -608,6 +610,19 @@ static void launch_iteration(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T
   }
 }
 
+// The iterations after q up to the next checkpoint (1-based iteration qc, a
+// multiple of replace_every) as one resident kernel, and the checkpoint's
+// kernels.  They return at once in a finished solve.
+template <typename T>
+static int launch_resident(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, T *const p[2], T *Ap,
+                           DevState *st, int q, int replace_every) {
+  const int qc = (q / replace_every + 1) * replace_every;
+  const int rc = bbpp_persist<T>(ctx, mask, r, p, Ap, x, st, replace_every);
+  launch_update<T>(ctx, r, Ap, st, 1);
+  launch_replace<T>(ctx, mask, x, rhs, r, p[qc & 1], st, RES_ITER);
+  return rc;
+}
+
 // Capture (or reuse) the graph of iterations q0+1 .. q0+len for these buffers.
 // Returns its index in ctx->graphs, or -1 after a CUDA error.
 // Capture len iterations (launch(i), i = 1 .. len) into a cached graph.
@@ -661,8 +676,9 @@ static int capture_chunk(bbpp_ctx *ctx, const GraphKey &key, int len, F launch, 
 
 template <typename T>
 static int get_chunk_graph(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, T *const p[2], T *Ap,
-                           DevState *st, int len, int replace_every, bool rr, cudaGraphExec_t *out) {
+                           DevState *st, int len, int replace_every, bool rr, bool resident, cudaGraphExec_t *out) {
   GraphKey key;
+  key.persist = resident;
   key.mask = mask;
   key.rhs = rhs;
   key.x = x;
@@ -679,6 +695,18 @@ static int get_chunk_graph(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *
   key.bscale = t_bscale;
   key.xhi = t_rel.xhi;
   key.rhs64 = t_rel.rhs;
+  if (resident) {
+    int rc = 0;
+    const int gi = capture_chunk(
+        ctx, key, len / replace_every,
+        [&](int i) {
+          const int rl =
+              launch_resident<T>(ctx, mask, rhs, x, r, p, Ap, st, (i - 1) * replace_every, replace_every);
+          if (rl) rc = rl;
+        },
+        out);
+    return rc ? -1 : gi;
+  }
   return capture_chunk(
       ctx, key, len, [&](int i) { launch_iteration<T>(ctx, mask, rhs, x, r, p, Ap, st, i, replace_every, rr); }, out);
 }
@@ -700,7 +728,11 @@ static int status_of(int done) {
 template <typename T>
 int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, T *const p[2], T *Ap, DevState *st,
                   DevState *hst, int replace_every, bool confirm, bool rr, int *iters_out) {
-  const int chunk = (replace_every % 2 == 0) ? replace_every : 2 * replace_every;
+  // resident iterations (grids that fit the chip): one kernel a checkpoint, so
+  // a graph holds four checkpoints; past the end of a solve a kernel takes ~2 us
+  const bool resident = bbpp_persist_ok(ctx, (int)sizeof(T));
+  const int chunk = resident ? 4 * replace_every : ((replace_every % 2 == 0) ? replace_every : 2 * replace_every);
+  if (resident && bbpp_persist_begin(ctx)) return BBPP_CUDA_ERROR;
   // q = completed iterations, read back from the device
   CK(cudaMemcpyAsync(hst, st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -719,7 +751,7 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
     std::vector<KEv> single;
     if (q % chunk == 0 && !ctx->profiling) {
       cudaGraphExec_t exec;
-      gi = get_chunk_graph<T>(ctx, mask, rhs, x, r, p, Ap, st, chunk, replace_every, rr, &exec);
+      gi = get_chunk_graph<T>(ctx, mask, rhs, x, r, p, Ap, st, chunk, replace_every, rr, resident, &exec);
       if (gi < 0) return BBPP_CUDA_ERROR;
       CK(cudaGraphLaunch(exec, ctx->stream));
       ctx->launches += ctx->graphs[gi].kernels;
@@ -733,6 +765,11 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
         ctx->launches += ((q + i) % replace_every == 0) ? 4 : 2;
       }
       ctx->rec = nullptr;
+      CK(cudaGetLastError());
+    } else if (resident) {
+      const int rl = launch_resident<T>(ctx, mask, rhs, x, r, p, Ap, st, q, replace_every);
+      if (rl) return rl;
+      ctx->launches += 4;
       CK(cudaGetLastError());
     } else {
       if (ctx->profiling) ctx->rec = &single;

@@ -68,6 +68,11 @@ struct DevState {
   double *trace_a;
   double *trace_b;
   int trace_n;
+  // pairs of FP32 iterations (bbpp_pair.cu): alpha and beta of both steps, the
+  // number of steps; residual kernels write z = r / dL in place of r
+  double pair[4];
+  int pair_steps;
+  int zform;
 };
 
 __device__ __forceinline__ void trace_put(double *buf, int n, int i, double v) {

@@ -797,6 +797,7 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
   // no predicated work on interior planes (FP64 issues at 1/64 of FP32).
   double corr = 0, rr = 0, bb = 0;
   const bool want_bb = mode == 0;
+  const bool zform = st->zform;  // write z = r / dL
   issue(z0 - 1);
   commit(0);
   issue(z0);
@@ -835,8 +836,7 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
       const TXT a = INTERIOR ? apply_L0<TXT, ISO>(G, pc, pe, pw, pn, ps, pt, pb, false)
                              : apply_L<TXT, ISO>(G, s_dL, cls, pc, pe, pw, pn, ps, pt, pb);
       const TXT rv = fma((TXT)bscale, bv, -a);
-      const TR ro = (TR)rv;
-      rout[c] = ro;
+      rout[c] = (!INTERIOR && zform) ? (TR)(rv * s_inv[cls]) : (TR)rv;
       const double rd = (double)rv;
       if (INTERIOR) {
         rr = fma(rd, rd, rr);
@@ -893,7 +893,7 @@ __device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3
     } else if (mode == 1) {
       st->replacements += 1;
       st->dlag = 0;  // x was settled before this residual
-      finish_iteration(st, rz1, rr1, true);
+      finish_iteration(st, rz1, rr1, !st->zform);  // a pair's kernels have counted theirs
       st->rr_ref = rr1;
       st->last_rep = st->iter;
     } else {  // confirm
@@ -999,6 +999,7 @@ __global__ void __launch_bounds__(FNT) k_resid_ff(const GeoL G, double *__restri
   };
   float corr = 0.f, rr = 0.f, bb = 0.f;
   const bool want_bb = mode == 0;
+  const bool zform = st->zform;  // write z = r / dL
   load_plane(0, z0 - 1);
   load_plane(1, z0);
   const int gx = x0 + tx;
@@ -1035,7 +1036,7 @@ __global__ void __launch_bounds__(FNT) k_resid_ff(const GeoL G, double *__restri
       const ff a = ff_add(d, ff_neg(s));
       const ff r = ff_add(ff_mul(bs, bv), ff_neg(a));
       const float rv = __fadd_rn(r.hi, r.lo);
-      rout[c] = rv;
+      rout[c] = zform ? rv * s_inv[cls] : rv;
       const float r2 = rv * rv;
       rr += r2;
       if (!INTERIOR && cls) corr = fmaf(s_inv[cls] - 1.f, r2, corr);

@@ -39,7 +39,7 @@ struct KEv {
 };
 
 enum KernelKind { KK_SEARCH_SPMV = 0, KK_UPDATE, KK_AXPY, KK_RESID, KK_SEARCH_SPMV_F32, KK_UPDATE_F32,
-                  KK_AXPY_F32, KK_RESID_F32, KK_FUSED_F32, KK_COUNT };
+                  KK_AXPY_F32, KK_RESID_F32, KK_FUSED_F32, KK_DOTS_F32, KK_COUNT };
 
 struct GraphCache {
   GraphKey key;
@@ -53,6 +53,7 @@ struct NetWork;     // learned-guess workspace (bbpp_net.cu)
 
 struct bbpp_tma_state;
 struct bbpp_persist_state;
+struct bbpp_pair_state;
 void *bbpp_tensor_map_encoder();  // cuTensorMapEncodeTiled, or null
 bool bbpp_tma_chunks(const bbpp_ctx *ctx, int *kz, int *nzc);  // z chunking of the TMA search kernel
 
@@ -92,6 +93,7 @@ struct bbpp_ctx {
   NetWork *net = nullptr;
   bbpp_tma_state *tma = nullptr;  // launch shape and tensor maps of the TMA search kernel
   bbpp_persist_state *persist = nullptr;  // boxes of the resident iteration (small grids)
+  bbpp_pair_state *pair = nullptr;        // launch shape of the paired FP32 iterations (large grids)
   bool pdl = false;               // iteration kernels launch with a programmatic dependency
   bool rev_update = true;         // the update kernel walks the search kernel's planes in reverse
   bool l2hint = true;             // FP32 iteration: mask evict_last in L2, p / Ap / x evict_first
@@ -199,6 +201,17 @@ bool bbpp_tma_fused(bbpp_ctx *ctx, const uint8_t *mask, const float *rin, const 
 bool bbpp_tma_search(bbpp_ctx *ctx, const uint8_t *mask, const float *r, const float *pold, float *pnew, float *Ap,
                      float *x, bbpp::DevState *st);
 int bbpp_residual_async(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs, const double *x, double *r);
+
+// two FP32 iterations as a dots and a step kernel (bbpp_pair.cu)
+void bbpp_pair_init(bbpp_ctx *ctx);
+void bbpp_pair_free(bbpp_ctx *ctx);
+bool bbpp_pair_ok(const bbpp_ctx *ctx);
+size_t bbpp_pair_partials(const bbpp_ctx *ctx);
+void bbpp_pair_launch(bbpp_ctx *ctx, bool step, const uint8_t *mask, const float *zin, const float *pin, float *zout,
+                      float *pout, float *x, bbpp::DevState *st, int replace_every);
+int bbpp_pcg_loop_pair(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, float *x, float *const z[2],
+                       float *const p[2], bbpp::DevState *st, bbpp::DevState *hst, int replace_every, bool confirm,
+                       int *iters_out);
 
 // iterations up to the next checkpoint in one resident kernel (bbpp_persist.cu)
 void bbpp_persist_init(bbpp_ctx *ctx);

@@ -80,6 +80,16 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   hst->wait_ns = ctx->wait_ns;
   hst->stop = o->stop;
   hst->first = 1;
+  // Pairs of iterations on grids of whole 16-byte rows (the mask is read in
+  // words), the resident iteration on grids that fit the chip.  Where both apply
+  // the line is at 3.2M cells: 144^3 (3.0M) took 27.9 us an iteration resident and
+  // 26.9 in pairs, 200x144x106 with walls (3.1M) 30.5 and 31.8, 160^3 (4.1M) 32.2
+  // and 30.7, 128^3 (2.1M) 21 and 23.
+  bool resident = bbpp_persist_ok(ctx, 4);
+  const bool pair =
+      ctx->fused && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 && (!resident || n > 3200000);
+  if (pair) resident = false;
+  hst->zform = pair ? 1 : 0;
   CK(cudaMemcpyAsync(st, hst, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(b->d, 0, sizeof(float) * n, ctx->stream));
   bbpp_launch_resid_s<double, float>(ctx, mask, x, rhs, b->rd, st, RES_INIT, S);
@@ -88,14 +98,19 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   bbpp_set_reliable(x, rhs);
   float *const p[2] = {b->p[0], b->p[1]};
   int it = 0;
-  bool fused = ctx->fused && bbpp_tma_fused_ok(ctx) && !bbpp_persist_ok(ctx, 4);
-  if (fused && !b->rd2) {
+  bool fused = ctx->fused && bbpp_tma_fused_ok(ctx) && !resident && !pair;
+  if (pair && !b->rd2) CK(cudaMalloc(&b->rd2, sizeof(float) * n));
+  if (fused && !b->Ap2) {
+    cudaFree(b->rd2);
+    b->rd2 = nullptr;
     CK(cudaMalloc(&b->rd2, sizeof(float) * n));
     CK(cudaMalloc(&b->Ap2, sizeof(float) * n));
   }
   float *const rs[2] = {b->rd, b->rd2}, *const as[2] = {b->Ap, b->Ap2};
   if (fused) fused = bbpp_tma_fused_maps(ctx, rs, as, p);
-  if (fused)
+  if (pair)
+    rc = bbpp_pcg_loop_pair(ctx, mask, b->r, b->d, rs, p, st, hst, o->replace_every, o->stop == BBPP_STOP_TRUE_REL, &it);
+  else if (fused)
     rc = bbpp_pcg_loop_fused(ctx, mask, b->r, b->d, rs, p, as, st, hst, o->replace_every,
                              o->stop == BBPP_STOP_TRUE_REL, &it);
   else

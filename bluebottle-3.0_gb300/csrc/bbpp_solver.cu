@@ -252,6 +252,7 @@ extern "C" int bbpp_create(const bbpp_grid *g, bbpp_ctx **out) {
   stencil_shape(ctx);
   bbpp_tma_init(ctx);
   bbpp_persist_init(ctx);
+  bbpp_pair_init(ctx);
   {
     // programmatic dependent launch of the iteration kernels: off unless
     // BBPP_PDL=1 (measured at 256^3: no gain, the kernels' own drain and fill
@@ -287,7 +288,7 @@ extern "C" int bbpp_create(const bbpp_grid *g, bbpp_ctx **out) {
                        (size_t)ctx->fgrid.x * ctx->fgrid.y * ctx->fgrid.z),
       std::max<size_t>(std::max<size_t>((size_t)ctx->pgrid[0].x * ctx->pgrid[0].y * ctx->pgrid[0].z,
                                         (size_t)ctx->pgrid[1].x * ctx->pgrid[1].y * ctx->pgrid[1].z),
-                       bbpp_tma_partials(ctx)));
+                       std::max(bbpp_pair_partials(ctx), bbpp_tma_partials(ctx))));
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
   ctx->stream = ctx->own_stream;
@@ -328,6 +329,7 @@ extern "C" int bbpp_destroy(bbpp_ctx *ctx) {
   bbpp_net_ctx_free(ctx);
   bbpp_tma_free(ctx);
   bbpp_persist_free(ctx);
+  bbpp_pair_free(ctx);
   if (ctx->st) cudaFree(ctx->st);
   if (ctx->trace) cudaFree(ctx->trace);
   if (ctx->partials) cudaFree(ctx->partials);
@@ -919,6 +921,105 @@ int bbpp_pcg_loop_fused(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, fl
   return 0;
 }
 
+// ----------------------------------------------------- paired iterations --
+// Pair k (from 0) reads z[k&1], p[k&1] twice and writes z[(k+1)&1], p[(k+1)&1];
+// x and z are current after each.  The host counts pairs (st->fq).
+static void launch_pair(bbpp_ctx *ctx, const uint8_t *mask, float *x, float *const z[2], float *const p[2],
+                        DevState *st, int k, int replace_every) {
+  const int i = k & 1, o = i ^ 1;
+  // bytes/cell: read z, p (+ mask); read z, p, x (+ mask), write z, p, x
+  bbpp_rec_begin(ctx, KK_DOTS_F32, 8.0 + (mask ? 1 : 0));
+  bbpp_pair_launch(ctx, false, mask, z[i], p[i], nullptr, nullptr, nullptr, st, replace_every);
+  bbpp_rec_end(ctx);
+  bbpp_rec_begin(ctx, KK_FUSED_F32, 24.0 + (mask ? 1 : 0));
+  bbpp_pair_launch(ctx, true, mask, z[i], p[i], z[o], p[o], x, st, replace_every);
+  bbpp_rec_end(ctx);
+}
+
+// The pairs from iteration it (pair k) up to the next checkpoint, and the
+// checkpoint's kernels (which return at once when it keeps the residual).
+static int launch_pairs(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, float *x, float *const z[2],
+                        float *const p[2], DevState *st, int it, int k, int replace_every) {
+  const int left = replace_every - it % replace_every, n = (left + 1) / 2;
+  for (int i = 0; i < n; i++) {
+    ctx->rec_iter = i + 1;
+    launch_pair(ctx, mask, x, z, p, st, k + i, replace_every);
+  }
+  launch_replace<float>(ctx, mask, x, rhs, z[(k + n) & 1], p[(k + n) & 1], st, RES_ITER);
+  return n;
+}
+
+int bbpp_pcg_loop_pair(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, float *x, float *const z[2],
+                       float *const p[2], DevState *st, DevState *hst, int replace_every, bool confirm,
+                       int *iters_out) {
+  // a graph holds an even count of pairs, so that it starts on the same buffers
+  const int per = (replace_every + 1) / 2, segments = per % 2 == 0 ? 1 : 2;
+  CK(cudaMemcpyAsync(p[0], z[0], sizeof(float) * (size_t)ctx->G.n, cudaMemcpyDeviceToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(hst, st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  long long rounds = 0;
+  const long long max_rounds = 4ll * (hst->max_iter / 1 + 2) + 64;
+  while (hst->done == RUNNING) {
+    if (++rounds > max_rounds) {
+      bbpp_record_error(ctx, cudaErrorUnknown, "solve loop made no progress", __LINE__);
+      return BBPP_CUDA_ERROR;
+    }
+    const int it0 = hst->iter, k0 = hst->fq;
+    std::vector<KEv> single;
+    if (it0 % replace_every == 0 && k0 % 2 == 0 && !ctx->profiling) {
+      GraphKey key;
+      key.mask = mask;
+      key.rhs = rhs;
+      key.x = x;
+      key.r = z[0];
+      key.r1 = z[1];
+      key.p0 = p[0];
+      key.p1 = p[1];
+      key.st = st;
+      key.len = 2 * per * segments;
+      key.replace_every = replace_every;
+      key.elem = 4;
+      key.stream = ctx->stream;
+      key.bscale = t_bscale;
+      key.xhi = t_rel.xhi;
+      key.rhs64 = t_rel.rhs;
+      cudaGraphExec_t exec;
+      const int gi = capture_chunk(
+          ctx, key, segments,
+          [&](int i) { launch_pairs(ctx, mask, rhs, x, z, p, st, 0, (i - 1) * per, replace_every); }, &exec);
+      if (gi < 0) return BBPP_CUDA_ERROR;
+      CK(cudaGraphLaunch(exec, ctx->stream));
+      ctx->launches += ctx->graphs[gi].kernels;
+    } else {
+      if (ctx->profiling) ctx->rec = &single;
+      ctx->launches += 2 * launch_pairs(ctx, mask, rhs, x, z, p, st, it0, k0, replace_every) + 2;
+      ctx->rec = nullptr;
+      CK(cudaGetLastError());
+    }
+    CK(cudaMemcpyAsync(hst, st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->profiling) bbpp_rec_collect(ctx, single, hst->fq - k0, true);
+    if (hst->done == DONE_PENDING) {
+      if (!confirm) {
+        hst->done = DONE_CONVERGED;
+        CK(cudaMemcpyAsync(&st->done, &hst->done, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+        break;
+      }
+      launch_replace<float>(ctx, mask, x, rhs, z[hst->fq & 1], p[hst->fq & 1], st, RES_CONFIRM);
+      ctx->launches += 2;
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(hst, st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
+      CK(cudaStreamSynchronize(ctx->stream));
+    }
+  }
+  // x into the FP64 solution, unless a replacement or confirmation came last
+  k_fold<<<ctx->egrid, FNT, 0, ctx->stream>>>(ctx->GL, t_rel.xhi, x, p[0], st, 0);
+  ctx->launches += 1;
+  CK(cudaGetLastError());
+  if (iters_out) *iters_out = hst->iter;
+  return 0;
+}
+
 template int bbpp_pcg_loop<double>(bbpp_ctx *, const uint8_t *, const double *, double *, double *, double *const[2],
                                    double *, DevState *, DevState *, int, bool, bool, int *);
 template int bbpp_pcg_loop<float>(bbpp_ctx *, const uint8_t *, const float *, float *, float *, float *const[2],
@@ -1465,7 +1566,7 @@ extern "C" int bbpp_stream_mix_rate(long long cells, double *bytes_per_s) {
 
 // ----------------------------------------------------------- kernel stats --
 static const char *kk_name[KK_COUNT] = {"search_spmv", "update", "axpy_x", "resid", "search_spmv_f32",
-                                        "update_f32", "axpy_x_f32", "resid_f32", "fused_f32"};
+                                        "update_f32", "axpy_x_f32", "resid_f32", "fused_f32", "dots_f32"};
 
 void bbpp_rec_begin(bbpp_ctx *ctx, int kind, double bytes_per_cell) {
   if (!ctx->rec) return;

@@ -229,11 +229,13 @@ typedef struct bbpp_kstat {
 } bbpp_kstat;
 int bbpp_kernel_stats(bbpp_ctx *ctx, bbpp_kstat *out, int max, int *n);
 /* Enable (1) or disable (0) per-kernel CUDA-event timing and reset the
- * counters; events are captured between the kernels of the graphs. */
+ * counters.  Kernels are timed one by one, so grids whose iterations run inside
+ * one launch (csrc/bbpp_persist.cu) take the kernels of single iterations. */
 int bbpp_set_profiling(bbpp_ctx *ctx, int on);
-/* The FP32 iteration of reliable-update solves: 1 = one fused kernel per
- * iteration (the default where the TMA kernels take the grid), 0 = a search
- * kernel and an update kernel. */
+/* The FP32 iteration of reliable-update solves on grids that do not fit the
+ * chip: 1 = pairs of iterations in two kernels (rows of a multiple of four
+ * cells up to 1024; the default), 0 = a search kernel and an update kernel per
+ * iteration. */
 int bbpp_set_fused(bbpp_ctx *ctx, int on);
 /* The outer residuals of the reliable updates (FP64 x into the FP32
  * residual): 0 = FP64 arithmetic (the default), 1 = float-float arithmetic on

@@ -15,8 +15,8 @@
 // Ap = 0 there.  A fluid cell's solid neighbour then contributes p = 0, which
 // is the reference's dropped off-diagonal (src/solver_kernel.cu:691-707).
 //
-//  k1_search2 p = invM r + beta p_old on a 64x16 tile plus halo (two cells per
-//             thread), ring of three planes in shared memory while the CTA
+//  k1_search2 p = invM r + beta p_old on a 64x8 tile plus halo (two cells per
+//             thread), ring of four planes in shared memory while the CTA
 //             marches in z; Ap = L p and the (p, Ap) partial.
 //  k2_update  r -= alpha Ap, (r,r) and the wall correction of (r,z), 16-byte
 //             vector loads; optionally in the reverse of the search kernel's
@@ -193,12 +193,16 @@ __host__ __device__ __forceinline__ bool xsum6(const double (&v)[6], double &out
 
 // The isotropic neighbour sum of FP64 p: xsum6 where it applies, FP64 adds in
 // the stencil's order otherwise.  A solid cell (`skip`) discards its result, so
-// it never takes the FP64 branch.
+// it never takes the FP64 branch.  The adds are a call: predicated into the
+// caller, they would occupy the FP64 pipe whether or not a lane takes them.
+__host__ __device__ __noinline__ static double nb_adds6(double pe, double pw, double pn, double ps, double pt, double pb) {
+  return ((pe + pw) + (pn + ps)) + (pt + pb);
+}
 __host__ __device__ __forceinline__ double nb_sum6(double pe, double pw, double pn, double ps, double pt, double pb,
                                           bool skip) {
   const double v[6] = {pe, pw, pn, ps, pt, pb};
   double s;
-  if (!xsum6(v, s)) s = skip ? 0.0 : ((pe + pw) + (pn + ps)) + (pt + pb);
+  if (!xsum6(v, s)) s = skip ? 0.0 : nb_adds6(pe, pw, pn, ps, pt, pb);
   return s;
 }
 
@@ -217,21 +221,27 @@ __device__ __forceinline__ double apply_L0<double, true>(const GeoL &G, double p
 
 // ------------------------------------------------------------ K1, pairs ---
 // K1, the search kernel: p_new = z + beta p_old (z = r on the scaled
-// operator) on the CTA's tile plus a one-cell halo, kept in a 3-plane shared
-// ring while the CTA marches in z; then Ap = L p_new and the (p, Ap) partial.
+// operator) on the CTA's tile plus a one-cell halo, kept in a 4-plane shared
+// ring while the CTA marches in z, one barrier a plane (the fourth plane spares the
+// second: a plane is overwritten two barriers after its last read, so the warps'
+// FP64 work on the next plane runs beside others' integer sums of this one); then Ap = L p_new and the (p, Ap) partial.
 // Replaces PP_update_search + exchange + PP_spmv_shared_load + thrust (p,Ap)
 // (src/solver_kernel.cu:528-713,906-927, src/cuda_solver.cu:201-205,256-263).
-// Two x-adjacent cells per thread: a tile is 64 x 16 cells (32 x 8 threads, two rows each).  Halo rows are loaded as aligned
+// Two x-adjacent cells per thread: a tile is 64 x 8 cells (32 x 8 threads, one row each).  Halo rows are loaded as aligned
 // pairs into shared rows padded so the pairs stay aligned (index 0 pad, 1 west
 // halo, 2..65 tile, 66 east halo); the two edge columns are scalar loads.
 // Only the thread's own cells need the mask (Ap = 0 in a solid cell), so it
 // is read straight from global memory.  Pairs need an even nx; odd nx uses
 // scalar loads.
 constexpr int PX = 64;          // tile width
-constexpr int PY = 16;          // tile height
+// rows a thread: one, so that four CTAs of 64 registers fit an SM (two rows and
+// three CTAs of 80 registers: 254 ms a plain FP64 solve at 256^3, against 244; five
+// CTAs spill: 285)
+constexpr int RPT = 1;
+constexpr int PY = 8 * RPT;     // tile height
 constexpr int PW = PX + 4;      // padded shared row
 constexpr int PHY = PY + 2;     // rows with halo
-constexpr int PROWS = (PHY + 7) / 8;  // halo rows per thread (3)
+constexpr int PROWS = (PHY + 7) / 8;  // halo rows per thread (2)
 
 template <typename T> struct V2of;
 template <> struct V2of<double> { typedef double2 type; };
@@ -261,13 +271,13 @@ __device__ __forceinline__ void store_own(T *__restrict__ pnew, T *__restrict__ 
 }
 
 template <typename T, bool MASK, bool ISO>
-__global__ void __launch_bounds__(FNT, sizeof(T) == 8 ? 3 : 4) k1_search2(const GeoL G, const T *__restrict__ r, const T *__restrict__ pold,
+__global__ void __launch_bounds__(FNT, 4) k1_search2(const GeoL G, const T *__restrict__ r, const T *__restrict__ pold,
                                                   T *__restrict__ pnew, T *__restrict__ Ap, T *__restrict__ x,
                                                   const uint8_t *__restrict__ mask, DevState *st, double *partials,
                                                   int kz) {
   typedef typename V2of<T>::type V2;
   __shared__ T s_dL[27], s_inv[27];
-  __shared__ __align__(16) T sp[3][PHY][PW];
+  __shared__ __align__(16) T sp[4][PHY][PW];
   __shared__ double s_red[FNT / 32];
   pdl_sync();
   if (*(volatile int *)&st->done) return;
@@ -422,23 +432,27 @@ __global__ void __launch_bounds__(FNT, sizeof(T) == 8 ? 3 : 4) k1_search2(const 
   commit(1, z0);
   issue(z0 + 1);
 
-  const int gy0 = y0 + ty, gy1 = y0 + ty + 8;
-  const bool m0 = npair > 0 && gy0 < ny, m1 = npair > 0 && gy1 < ny;
-  const int cy0 = m0 ? 3 * wall_count(gy0, ny, G.py) : 0;
-  const int cy1 = m1 ? 3 * wall_count(gy1, ny, G.py) : 0;
+  int gyh[RPT], cyh[RPT];
+  bool mh[RPT];
+#pragma unroll
+  for (int h = 0; h < RPT; h++) {
+    gyh[h] = y0 + ty + 8 * h;
+    mh[h] = npair > 0 && gyh[h] < ny;
+    cyh[h] = mh[h] ? 3 * wall_count(gyh[h], ny, G.py) : 0;
+  }
   typename Acc<T>::type acc = 0;
 
   for (int z = z0; z < z1; z++) {
-    const int sb = (z - z0) % 3, sc = (z - z0 + 1) % 3, st_ = (z - z0 + 2) % 3;
+    const int sb = (z - z0) & 3, sc = (z - z0 + 1) & 3, st_ = (z - z0 + 2) & 3;
     commit(st_, z + 1);
     if (z + 2 <= z1) issue(z + 2);
     // own-cell mask of this plane (used after the barrier)
-    uint8_t mk[2][2] = {{0, 0}, {0, 0}};
+    uint8_t mk[RPT][2] = {};
     if (MASK) {
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        if (!(h ? m1 : m0)) continue;
-        const unsigned int c = plane * (unsigned int)z + (unsigned int)nx * (unsigned int)(h ? gy1 : gy0) + gxp;
+      for (int h = 0; h < RPT; h++) {
+        if (!mh[h]) continue;
+        const unsigned int c = plane * (unsigned int)z + (unsigned int)nx * (unsigned int)gyh[h] + gxp;
         if (pair_full) {
           const uchar2 mm = *reinterpret_cast<const uchar2 *>(mask + c);
           mk[h][0] = mm.x;
@@ -453,8 +467,8 @@ __global__ void __launch_bounds__(FNT, sizeof(T) == 8 ? 3 : 4) k1_search2(const 
     const int wz = 9 * wall_count(z, nz, G.pz);
     const bool interior = !xy_walls && wz == 0;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if (!(h ? m1 : m0)) continue;
+    for (int h = 0; h < RPT; h++) {
+      if (!mh[h]) continue;
       const int ly = ty + 1 + 8 * h;
       const int col = 2 + 2 * tx;
       const V2 c = *reinterpret_cast<const V2 *>(&sp[sc][ly][col]);
@@ -468,7 +482,7 @@ __global__ void __launch_bounds__(FNT, sizeof(T) == 8 ? 3 : 4) k1_search2(const 
         a0 = apply_L0<T, ISO>(G, c.x, c.y, w, n.x, s.x, t.x, b.x, MASK && mk[h][0]);
         a1 = apply_L0<T, ISO>(G, c.y, e, c.x, n.y, s.y, t.y, b.y, MASK && mk[h][1]);
       } else {
-        const int cy = (h ? cy1 : cy0) + wz;
+        const int cy = cyh[h] + wz;
         a0 = apply_L<T, ISO>(G, s_dL, wxp0 + cy, c.x, c.y, w, n.x, s.x, t.x, b.x);
         a1 = apply_L<T, ISO>(G, s_dL, wxp1 + cy, c.y, e, c.x, n.y, s.y, t.y, b.y);
       }
@@ -476,7 +490,7 @@ __global__ void __launch_bounds__(FNT, sizeof(T) == 8 ? 3 : 4) k1_search2(const 
         if (mk[h][0]) a0 = T(0);
         if (mk[h][1]) a1 = T(0);
       }
-      const unsigned int cc = plane * (unsigned int)z + (unsigned int)nx * (unsigned int)(h ? gy1 : gy0) + gxp;
+      const unsigned int cc = plane * (unsigned int)z + (unsigned int)nx * (unsigned int)gyh[h] + gxp;
       if (pair_full) {
         V2 o;
         o.x = a0;
@@ -493,7 +507,6 @@ __global__ void __launch_bounds__(FNT, sizeof(T) == 8 ? 3 : 4) k1_search2(const 
         }
       }
     }
-    __syncthreads();
   }
   double v[1] = {(double)acc}, tot[1];
   const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
@@ -737,8 +750,8 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
                                                  TR *__restrict__ rout, const uint8_t *__restrict__ mask,
                                                  DevState *st, double *partials, int kz, int mode, double bscale) {
   __shared__ TXT s_dL[27], s_inv[27];
-  __shared__ TXT sp[3][FHY][FHX];
-  __shared__ uint8_t sm[3][FHY][FHX + 2];
+  __shared__ TXT sp[4][FHY][FHX];
+  __shared__ uint8_t sm[4][FHY][FHX + 2];
   __shared__ double s_red[3 * FNT / 32];
   pdl_sync();
   if (mode == 1 && skip_step(st, 2)) return;
@@ -850,14 +863,13 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
   TXT bcur[2] = {TXT(0), TXT(0)}, bnext[2] = {TXT(0), TXT(0)};
   if (z0 < z1) load_b(z0, bcur);
   for (int z = z0; z < z1; z++) {
-    const int sb = (z - z0) % 3, sc = (z - z0 + 1) % 3, st_ = (z - z0 + 2) % 3;
+    const int sb = (z - z0) & 3, sc = (z - z0 + 1) & 3, st_ = (z - z0 + 2) & 3;
     commit(st_);  // plane z + 1, loaded during the previous plane
     if (z + 2 <= z1) issue(z + 2);
     if (z + 1 < z1) load_b(z + 1, bnext);
     __syncthreads();
     if (G.px && G.py && wall_count(z, nz, G.pz) == 0) cell(std::true_type(), sb, sc, st_, z, bcur);
     else cell(std::false_type(), sb, sc, st_, z, bcur);
-    __syncthreads();
     bcur[0] = bnext[0];
     bcur[1] = bnext[1];
   }

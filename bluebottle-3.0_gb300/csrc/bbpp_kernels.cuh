@@ -15,6 +15,7 @@
 #pragma once
 
 #include "bbpp_dev.cuh"
+#include "bbpp_fast.cuh"
 
 namespace bbpp {
 
@@ -23,6 +24,7 @@ constexpr int TY = 8;   // tile height (y)
 constexpr int HX = TX + 2;
 constexpr int HY = TY + 2;
 constexpr int NT = TX * TY;  // 256 threads
+constexpr int HPER = (HX * HY + NT - 1) / NT;  // halo elements per thread
 
 enum ResidMode : int { RES_INIT = 0, RES_ITER = 1, RES_CONFIRM = 2, RES_PLAIN = 3 };
 
@@ -39,17 +41,25 @@ __global__ void __launch_bounds__(NT) k_axpy_x(const Geo G, T *__restrict__ x, c
   for (unsigned int c = blockIdx.x * NT + threadIdx.x; c < n; c += gridDim.x * NT) x[c] = fma(alpha, p[c], x[c]);
 }
 
+// rz + w rd^2: a wall cell's part of (r,z), as a call (see nb_adds6)
+__device__ __noinline__ static double wall_rz(double rz, double w, double rd) { return fma(rd, w * rd, rz); }
+
 // ------------------------------------------------------------ residual -----
 // r = rhs - (-A) x   (rhs != NULL), or r = (-A) x  (rhs == NULL, RES_PLAIN).
 // TX: type of x and rhs; TR: type of r.  Partials: (r,z), (r,r), (rhs,rhs).
+// xsum (FP64, cx == cy == cz): the six neighbours, zero across solid cells and
+// walls, as one exact sum on the integer pipe (xsum6).
+// Bound by the FP64 pipe with FP64 adds (13 instructions a cell; 426 us at 256^3);
+// with the integer sums, (r,z) as (r,r) plus the wall cells' part, and a plane's
+// loads in flight while the one before is computed it takes 276 us.
 template <typename TXT, typename TR, bool MASK>
 __global__ void __launch_bounds__(NT) k_resid(const Geo G, const TXT *__restrict__ xin,
                                               const TXT *__restrict__ rhs, TR *__restrict__ rout,
                                               const uint8_t *__restrict__ mask, DevState *st,
-                                              double *partials, int kz, int mode) {
+                                              double *partials, int kz, int mode, int xsum) {
   __shared__ double s_tab[81];
-  __shared__ TXT sp[3][HY][HX];
-  __shared__ uint8_t sm[3][HY][HX + 2];
+  __shared__ TXT sp[4][HY][HX];
+  __shared__ uint8_t sm[4][HY][HX + 2];
   __shared__ double s_red[3 * NT / 32];
   if (mode == RES_ITER && *(volatile int *)&st->done) return;
   load_tab(G, s_tab);
@@ -61,33 +71,57 @@ __global__ void __launch_bounds__(NT) k_resid(const Geo G, const TXT *__restrict
   const int nx = G.nx, ny = G.ny, nz = G.nz;
   __syncthreads();
 
-  auto load_plane = [&](int slot, int zr) {
+  // the tile of a plane plus halo: loaded into registers one plane ahead (issue),
+  // written to shared memory the next plane (commit)
+  long long eoff[HPER];  // offset in a plane, -1 outside a wall or the tile
+#pragma unroll
+  for (int k = 0; k < HPER; k++) {
+    const int e = tid + k * NT, ly = e / HX, lx = e - ly * HX;
+    const int hx = halo_index(x0 + lx - 1, nx, G.px), hy = halo_index(y0 + ly - 1, ny, G.py);
+    eoff[k] = e < HX * HY && hx >= 0 && hy >= 0 ? hx + (long long)nx * hy : -1;
+  }
+  TXT pv[HPER];
+  uint8_t pm[HPER];
+  auto issue = [&](int zr) {
     const int gz = halo_index(zr, nz, G.pz);
-    for (int e = tid; e < HX * HY; e += NT) {
-      const int ly = e / HX, lx = e - ly * HX;
-      const int gx = halo_index(x0 + lx - 1, nx, G.px), gy = halo_index(y0 + ly - 1, ny, G.py);
-      TXT val = TXT(0);
-      uint8_t m = 0;
-      if (gz >= 0 && gx >= 0 && gy >= 0) {
-        const long long c = gx + (long long)nx * (gy + (long long)ny * gz);
-        val = xin[c];
-        if (MASK) m = mask[c];
+#pragma unroll
+    for (int k = 0; k < HPER; k++) {
+      pv[k] = TXT(0);
+      pm[k] = 0;
+      if (gz >= 0 && eoff[k] >= 0) {
+        const long long c = eoff[k] + (long long)nx * ny * gz;
+        pv[k] = xin[c];
+        if (MASK) pm[k] = mask[c];
       }
-      sp[slot][ly][lx] = val;
-      sm[slot][ly][lx] = m;
+    }
+  };
+  auto commit = [&](int slot) {
+#pragma unroll
+    for (int k = 0; k < HPER; k++) {
+      const int e = tid + k * NT;
+      if (e >= HX * HY) continue;
+      (&sp[slot][0][0])[e] = pv[k];
+      const int ly = e / HX;
+      sm[slot][ly][e - ly * HX] = pm[k];
     }
   };
 
   double rz = 0, rr = 0, bb = 0;
-  load_plane(0, z0 - 1);
-  load_plane(1, z0);
+  issue(z0 - 1);
+  commit(0);
+  issue(z0);
+  commit(1);
+  issue(z0 + 1);
   const TXT cx = (TXT)G.cx, cy = (TXT)G.cy, cz = (TXT)G.cz;
   const int gx = x0 + tx, gy = y0 + ty;
   const bool mine = gx < nx && gy < ny;
   const int cls_xy = mine ? (wall_count(gx, nx, G.px) + 3 * wall_count(gy, ny, G.py)) : 0;
   for (int z = z0; z < z1; z++) {
-    const int sb = (z - z0) % 3, sc = (z - z0 + 1) % 3, st_ = (z - z0 + 2) % 3;
-    load_plane(st_, z + 1);
+    const int sb = (z - z0) & 3, sc = (z - z0 + 1) & 3, st_ = (z - z0 + 2) & 3;
+    commit(st_);
+    if (z + 2 <= z1) issue(z + 2);
+    const long long c = gx + (long long)nx * (gy + (long long)ny * z);
+    const TXT bv = rhs && mine ? rhs[c] : TXT(0);
     __syncthreads();
     if (mine) {
       TXT pc = sp[sc][ty + 1][tx + 1];
@@ -106,28 +140,30 @@ __global__ void __launch_bounds__(NT) k_resid(const Geo G, const TXT *__restrict
         pb = (mc || sm[sb][ty + 1][tx + 1]) ? TXT(0) : pb;
         d = mc ? (TXT)s_tab[54 + cls] : d;
       }
-      TXT s = cx * (pe + pw);
-      s = fma(cy, pn + ps, s);
-      s = fma(cz, pt + pb, s);
-      const TXT a = fma(d, pc, -s);
-      const long long c = gx + (long long)nx * (gy + (long long)ny * z);
+      TXT a;
+      if (sizeof(TXT) == 8 && xsum) {
+        a = fma(-cx, (TXT)nb_sum6(pe, pw, pn, ps, pt, pb, false), d * pc);
+      } else {
+        TXT s = cx * (pe + pw);
+        s = fma(cy, pn + ps, s);
+        s = fma(cz, pt + pb, s);
+        a = fma(d, pc, -s);
+      }
       if (rhs) {
-        const TXT bv = rhs[c];
         const TXT rv = bv - a;
         const TR ro = (TR)rv;
         rout[c] = ro;
         const double rd = (double)rv;
-        rz = fma(rd, s_tab[27 + cls] * rd, rz);
         rr = fma(rd, rd, rr);
+        if (cls) rz = wall_rz(rz, s_tab[27 + cls] - s_tab[27], rd);
         bb = fma((double)bv, (double)bv, bb);
       } else {
         rout[c] = (TR)a;
       }
     }
-    __syncthreads();
   }
   if (mode == RES_PLAIN) return;
-  double v[3] = {rz, rr, bb}, tot[3];
+  double v[3] = {fma(s_tab[27], rr, rz), rr, bb}, tot[3];
   const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
   const unsigned int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
   if (last_cta_reduce<3>(v, partials, st, nb, bid, s_red, tot) && tid == 0) {

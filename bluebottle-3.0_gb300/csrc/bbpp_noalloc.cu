@@ -89,12 +89,13 @@ extern "C" int bbpp_residual_noalloc(const bbpp_grid *g, const uint8_t *mask, co
   NoallocScratch *sc = reinterpret_cast<NoallocScratch *>(base);
   cudaStream_t s = (cudaStream_t)stream;
   // the solver state (ticket counter, thresholds) must start at zero
+  const int xsum = G.cx == G.cy && G.cy == G.cz;
   cudaError_t e = cudaMemsetAsync(&sc->st, 0, sizeof(DevState), s);
   if (e == cudaSuccess) {
     if (mask)
-      k_resid<double, double, true><<<grid, NT, 0, s>>>(G, x, rhs, r, mask, &sc->st, sc->partials, kz, RES_INIT);
+      k_resid<double, double, true><<<grid, NT, 0, s>>>(G, x, rhs, r, mask, &sc->st, sc->partials, kz, RES_INIT, xsum);
     else
-      k_resid<double, double, false><<<grid, NT, 0, s>>>(G, x, rhs, r, mask, &sc->st, sc->partials, kz, RES_INIT);
+      k_resid<double, double, false><<<grid, NT, 0, s>>>(G, x, rhs, r, mask, &sc->st, sc->partials, kz, RES_INIT, xsum);
     e = cudaGetLastError();
   }
   DevState h;

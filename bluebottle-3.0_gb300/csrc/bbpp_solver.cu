@@ -133,49 +133,89 @@ __global__ void k_invm(const Geo G, double *invM) {
   }
 }
 
-// Sphere phase mask (build_phase, src/particle_kernel.cu:148-253).  One CTA
-// per (sphere, periodic image) walks the image's bounding box and marks the
+// Sphere phase mask (build_phase, src/particle_kernel.cu:148-253).  A CTA per
+// sphere: the lanes of its first warp find the bounding boxes of the sphere's
+// periodic images, then all threads walk the boxes that meet the grid and mark the
 // cells whose centre satisfies floor(d/r) < 1.  The mask must be zeroed first.
-// Products and sums use round-to-nearest intrinsics (no FMA contraction) so
-// the result is bit-identical to the host restatement.
-__global__ void k_sphere_mask(const Geo G, double dx, double dy, double dz, double xs, double ys,
-                              double zs, int nimg_x, int nimg_y, int nimg_z,
-                              const Sphere *__restrict__ sph, uint8_t *mask) {
+// Products and sums of that test use round-to-nearest intrinsics (no FMA
+// contraction) so the result is bit-identical to the host restatement; cells that
+// FP32 places clearly inside or outside (all but those within its error of the
+// surface) skip it.  Bound by the FP64 pipe before: a CTA per image, whose 256
+// threads each found its box and tested every cell in FP64, took 630 us for 1000
+// spheres of radius 6 at 256^3; this takes 17.
+struct SphereBox {
+  int i0, j0, k0, bx, by, n;  // n = 0: no cell of the grid
+  double X, Y, Z;             // centre less the origin
+  float fx, fy, fz;           // the first cell's centre from the sphere's
+};
+
+__global__ void __launch_bounds__(256) k_sphere_mask(const Geo G, double dx, double dy, double dz, double xs,
+                                                     double ys, double zs, int nimg_x, int nimg_y, int nimg_z,
+                                                     const Sphere *__restrict__ sph, uint8_t *mask) {
+  __shared__ SphereBox s_box[27];
   const int nimg = nimg_x * nimg_y * nimg_z;
-  const int s = blockIdx.x / nimg;
-  int im = blockIdx.x - s * nimg;
-  const int ox = (nimg_x == 3) ? (im % 3) - 1 : 0;
-  im /= nimg_x;
-  const int oy = (nimg_y == 3) ? (im % 3) - 1 : 0;
-  im /= nimg_y;
-  const int oz = (nimg_z == 3) ? im - 1 : 0;
-  const Sphere S = sph[s];
+  const Sphere S = sph[blockIdx.x];
+  if (threadIdx.x < nimg) {
+    int im = threadIdx.x;
+    const int ox = (nimg_x == 3) ? (im % 3) - 1 : 0;
+    im /= nimg_x;
+    const int oy = (nimg_y == 3) ? (im % 3) - 1 : 0;
+    im /= nimg_y;
+    const int oz = (nimg_z == 3) ? im - 1 : 0;
+    const double X = __dadd_rn(S.x, __dmul_rn((double)ox, __dmul_rn((double)G.nx, dx)));
+    const double Y = __dadd_rn(S.y, __dmul_rn((double)oy, __dmul_rn((double)G.ny, dy)));
+    const double Z = __dadd_rn(S.z, __dmul_rn((double)oz, __dmul_rn((double)G.nz, dz)));
+    SphereBox b;
+    b.X = __dsub_rn(X, xs);
+    b.Y = __dsub_rn(Y, ys);
+    b.Z = __dsub_rn(Z, zs);
+    int i0 = (int)floor(__ddiv_rn(__dsub_rn(b.X, S.w), dx)) - 1;
+    int i1 = (int)ceil(__ddiv_rn(__dadd_rn(b.X, S.w), dx)) + 1;
+    int j0 = (int)floor(__ddiv_rn(__dsub_rn(b.Y, S.w), dy)) - 1;
+    int j1 = (int)ceil(__ddiv_rn(__dadd_rn(b.Y, S.w), dy)) + 1;
+    int k0 = (int)floor(__ddiv_rn(__dsub_rn(b.Z, S.w), dz)) - 1;
+    int k1 = (int)ceil(__ddiv_rn(__dadd_rn(b.Z, S.w), dz)) + 1;
+    i0 = max(i0, 0); j0 = max(j0, 0); k0 = max(k0, 0);
+    i1 = min(i1, G.nx - 1); j1 = min(j1, G.ny - 1); k1 = min(k1, G.nz - 1);
+    b.i0 = i0;
+    b.j0 = j0;
+    b.k0 = k0;
+    b.bx = i1 - i0 + 1;
+    b.by = j1 - j0 + 1;
+    b.n = i1 < i0 || j1 < j0 || k1 < k0 ? 0 : b.bx * b.by * (k1 - k0 + 1);
+    b.fx = (float)(((double)(i0 + 1) - 0.5) * dx - b.X);
+    b.fy = (float)(((double)(j0 + 1) - 0.5) * dy - b.Y);
+    b.fz = (float)(((double)(k0 + 1) - 0.5) * dz - b.Z);
+    s_box[threadIdx.x] = b;
+  }
+  __syncthreads();
   const double irad = 1.0 / S.w;
-  const double X = __dadd_rn(S.x, __dmul_rn((double)ox, __dmul_rn((double)G.nx, dx)));
-  const double Y = __dadd_rn(S.y, __dmul_rn((double)oy, __dmul_rn((double)G.ny, dy)));
-  const double Z = __dadd_rn(S.z, __dmul_rn((double)oz, __dmul_rn((double)G.nz, dz)));
-  int i0 = (int)floor(__ddiv_rn(__dsub_rn(__dsub_rn(X, xs), S.w), dx)) - 1;
-  int i1 = (int)ceil(__ddiv_rn(__dadd_rn(__dsub_rn(X, xs), S.w), dx)) + 1;
-  int j0 = (int)floor(__ddiv_rn(__dsub_rn(__dsub_rn(Y, ys), S.w), dy)) - 1;
-  int j1 = (int)ceil(__ddiv_rn(__dadd_rn(__dsub_rn(Y, ys), S.w), dy)) + 1;
-  int k0 = (int)floor(__ddiv_rn(__dsub_rn(__dsub_rn(Z, zs), S.w), dz)) - 1;
-  int k1 = (int)ceil(__ddiv_rn(__dadd_rn(__dsub_rn(Z, zs), S.w), dz)) + 1;
-  i0 = max(i0, 0); j0 = max(j0, 0); k0 = max(k0, 0);
-  i1 = min(i1, G.nx - 1); j1 = min(j1, G.ny - 1); k1 = min(k1, G.nz - 1);
-  if (i1 < i0 || j1 < j0 || k1 < k0) return;
-  const int bx = i1 - i0 + 1, by = j1 - j0 + 1, bz = k1 - k0 + 1;
-  const int nbox = bx * by * bz;
-  const double Xs = __dsub_rn(X, xs), Ys = __dsub_rn(Y, ys), Zs = __dsub_rn(Z, zs);
-  for (int e = threadIdx.x; e < nbox; e += blockDim.x) {
-    const int li = e % bx, t = e / bx;
-    const int lj = t % by, lk = t / by;
-    const int i = i0 + li, j = j0 + lj, k = k0 + lk;
-    const double xx = __dsub_rn(__dmul_rn((double)(i + 1) - 0.5, dx), Xs);
-    const double yy = __dsub_rn(__dmul_rn((double)(j + 1) - 0.5, dy), Ys);
-    const double zz = __dsub_rn(__dmul_rn((double)(k + 1) - 0.5, dz), Zs);
-    const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(xx, xx), __dmul_rn(yy, yy)), __dmul_rn(zz, zz));
-    const double d = __dsqrt_rn(d2);
-    if (floor(__dmul_rn(d, irad)) < 1.0) mask[i + (long long)G.nx * (j + (long long)G.ny * k)] = 1;
+  const float fdx = (float)dx, fdy = (float)dy, fdz = (float)dz, fr2 = (float)S.w * (float)S.w;
+  // A box reaches r + 2 dx from the centre; a coordinate's FP32 error there is below
+  // 3 * 2^-23 of that, the squared distance's below 2 sqrt(3) times as much of its
+  // square and a few roundings.  Twice that; no FP32 decision where squares leave
+  // its normal range.
+  const float reach = (float)S.w + 3.f * fmaxf(fdx, fmaxf(fdy, fdz));
+  const float near = fr2 > 1e-30f && reach < 1e18f ? 4e-6f * reach * reach : __int_as_float(0x7f800000);
+  for (int im = 0; im < nimg; im++) {
+    const SphereBox &b = s_box[im];
+    for (int e = threadIdx.x; e < b.n; e += 256) {
+      const int li = e % b.bx, t = e / b.bx;
+      const int lj = t % b.by, lk = t / b.by;
+      const int i = b.i0 + li, j = b.j0 + lj, k = b.k0 + lk;
+      const float fx = fmaf((float)li, fdx, b.fx), fy = fmaf((float)lj, fdy, b.fy), fz = fmaf((float)lk, fdz, b.fz);
+      const float over = fmaf(fx, fx, fmaf(fy, fy, fz * fz)) - fr2;
+      if (over > near) continue;
+      bool inside = over < -near;
+      if (!inside) {
+        const double xx = __dsub_rn(__dmul_rn((double)(i + 1) - 0.5, dx), b.X);
+        const double yy = __dsub_rn(__dmul_rn((double)(j + 1) - 0.5, dy), b.Y);
+        const double zz = __dsub_rn(__dmul_rn((double)(k + 1) - 0.5, dz), b.Z);
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(xx, xx), __dmul_rn(yy, yy)), __dmul_rn(zz, zz));
+        inside = floor(__dmul_rn(__dsqrt_rn(d2), irad)) < 1.0;
+      }
+      if (inside) mask[i + (long long)G.nx * (j + (long long)G.ny * k)] = 1;
+    }
   }
 }
 
@@ -332,6 +372,7 @@ extern "C" int bbpp_destroy(bbpp_ctx *ctx) {
   bbpp_pair_free(ctx);
   if (ctx->st) cudaFree(ctx->st);
   if (ctx->trace) cudaFree(ctx->trace);
+  if (ctx->sph) cudaFree(ctx->sph);
   if (ctx->partials) cudaFree(ctx->partials);
   if (ctx->r) cudaFree(ctx->r);
   if (ctx->p[0]) cudaFree(ctx->p[0]);
@@ -472,12 +513,13 @@ static void launch_update(bbpp_ctx *ctx, T *r, const T *Ap, DevState *st, int co
 template <typename TXT, typename TR>
 static void launch_resid(bbpp_ctx *ctx, const uint8_t *mask, const TXT *x, const TXT *rhs, TR *r, DevState *st,
                          int mode) {
+  const int xsum = ctx->GL.iso && ctx->GL.xsum;
   if (mask)
     k_resid<TXT, TR, true><<<ctx->sgrid, NT, 0, ctx->stream>>>(ctx->G, x, rhs, r, mask, st, ctx->partials, ctx->kz,
-                                                               mode);
+                                                               mode, xsum);
   else
     k_resid<TXT, TR, false><<<ctx->sgrid, NT, 0, ctx->stream>>>(ctx->G, x, rhs, r, mask, st, ctx->partials,
-                                                                ctx->kz, mode);
+                                                                ctx->kz, mode, xsum);
 }
 
 template <typename TXT, typename TR>
@@ -1209,21 +1251,40 @@ extern "C" int bbpp_invm(bbpp_ctx *ctx, double *invM) {
   return 0;
 }
 
+// v * m rounded to nearest.  Where m is 2^k (k != none) by adding k to the exponent
+// on the integer pipe; zero, subnormal, infinite and NaN v and results out of the
+// normal range take the multiplication.
+// That branch is a call: predicated, an FP64 instruction occupies the pipe whether
+// or not a lane takes it.
+constexpr int kNoPow2 = 1 << 20;
+__device__ __noinline__ double mul_call(double v, double m) { return __dmul_rn(v, m); }
+__device__ __forceinline__ double mul_pow2(double v, double m, int k) {
+  const int hi = __double2hiint(v);
+  const unsigned int e = (unsigned int)(hi >> 20) & 0x7ffu;
+  if (k == kNoPow2 || e == 0u || e == 0x7ffu || (int)e + k < 1 || (int)e + k > 2046)
+    return mul_call(v, m);
+  return __hiloint2double(hi + (k << 20), __double2loint(v));
+}
+
 // PP_rhs (src/solver_kernel.cu:152-173) on dense face arrays: rhs = -(rho/dt)
-// div u*, the reference's evaluation order without contraction.
-__global__ void k_rhs_div(int nx, int ny, int nz, double idx, double idy, double idz, double rho_idt,
-                          const double *__restrict__ u, const double *__restrict__ v, const double *__restrict__ w,
-                          double *__restrict__ rhs) {
-  const long long n = (long long)nx * ny * nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % nx);
-    const long long r = c / nx;
-    const int j = (int)(r % ny), k = (int)(r / ny);
-    const long long uw = i + (long long)(nx + 1) * (j + (long long)ny * k);
-    const long long vs = i + (long long)nx * (j + (long long)(ny + 1) * k);
-    double s = __dmul_rn(__dsub_rn(u[uw + 1], u[uw]), idx);
-    s = __dadd_rn(s, __dmul_rn(__dsub_rn(v[vs + nx], v[vs]), idy));
-    s = __dadd_rn(s, __dmul_rn(__dsub_rn(w[c + (long long)nx * ny], w[c]), idz));
+// div u*, the reference's evaluation order without contraction.  Bound by the FP64
+// pipe (9 instructions a cell); on spacings of 1 / 2^k, the usual ones, six
+// (POW2): at 256^3 333 us before, 205 now.
+template <bool POW2>
+__global__ void __launch_bounds__(256) k_rhs_div(const Geo G, double idx, double idy, double idz, int kx, int ky,
+                                                 int kz, double rho_idt, const double *__restrict__ u,
+                                                 const double *__restrict__ v, const double *__restrict__ w,
+                                                 double *__restrict__ rhs) {
+  const unsigned int n = (unsigned int)G.n;
+  const size_t plane = (size_t)G.nx * G.ny;
+  for (unsigned int c = blockIdx.x * 256u + threadIdx.x; c < n; c += gridDim.x * 256u) {
+    const unsigned int row = fdiv(c, G.mx), k = fdiv(c, G.mxy);
+    const size_t uw = (size_t)c + row, vs = (size_t)c + (size_t)G.nx * k;
+    const double du = __dsub_rn(u[uw + 1], u[uw]), dv = __dsub_rn(v[vs + G.nx], v[vs]),
+                 dw = __dsub_rn(w[c + plane], w[c]);
+    double s = POW2 ? mul_pow2(du, idx, kx) : __dmul_rn(du, idx);
+    s = __dadd_rn(s, POW2 ? mul_pow2(dv, idy, ky) : __dmul_rn(dv, idy));
+    s = __dadd_rn(s, POW2 ? mul_pow2(dw, idz, kz) : __dmul_rn(dw, idz));
     rhs[c] = -__dmul_rn(s, rho_idt);
   }
 }
@@ -1232,8 +1293,18 @@ extern "C" int bbpp_rhs_div(bbpp_ctx *ctx, double rho_f, double dt, const double
                             double *rhs) {
   if (!ctx || !u || !v || !w || !rhs || !(dt != 0.0)) return BBPP_BAD_ARG;
   const Geo &G = ctx->G;
-  k_rhs_div<<<ctx->egrid, NT, 0, ctx->stream>>>(G.nx, G.ny, G.nz, 1. / ctx->grid.dx, 1. / ctx->grid.dy,
-                                                 1. / ctx->grid.dz, rho_f / dt, u, v, w, rhs);
+  const double id[3] = {1. / ctx->grid.dx, 1. / ctx->grid.dy, 1. / ctx->grid.dz};
+  int k[3];
+  for (int a = 0; a < 3; a++) {
+    int e;
+    k[a] = std::frexp(id[a], &e) == 0.5 && e > -1000 && e < 1000 ? e - 1 : kNoPow2;
+  }
+  if (k[0] != kNoPow2 || k[1] != kNoPow2 || k[2] != kNoPow2)
+    k_rhs_div<true><<<ctx->egrid, 256, 0, ctx->stream>>>(G, id[0], id[1], id[2], k[0], k[1], k[2], rho_f / dt, u, v, w,
+                                                         rhs);
+  else
+    k_rhs_div<false><<<ctx->egrid, 256, 0, ctx->stream>>>(G, id[0], id[1], id[2], k[0], k[1], k[2], rho_f / dt, u, v, w,
+                                                          rhs);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return 0;
@@ -1347,16 +1418,21 @@ extern "C" int bbpp_sphere_mask(bbpp_ctx *ctx, double xs, double ys, double zs, 
     if (!(rad[s] > 0)) return BBPP_BAD_ARG;
     h[s] = Sphere{cx[s], cy[s], cz[s], rad[s]};
   }
-  Sphere *d = nullptr;
-  CK(cudaMalloc(&d, sizeof(Sphere) * nsph));
+  // the context keeps the spheres' buffer (making one a call took ~100 us)
+  if (ctx->sph_cap < nsph) {
+    cudaFree(ctx->sph);
+    ctx->sph = nullptr;
+    ctx->sph_cap = 0;
+    CK(cudaMalloc(&ctx->sph, sizeof(Sphere) * nsph));
+    ctx->sph_cap = nsph;
+  }
+  Sphere *d = (Sphere *)ctx->sph;
   CK(cudaMemcpyAsync(d, h.data(), sizeof(Sphere) * nsph, cudaMemcpyHostToDevice, ctx->stream));
   const int ix = ctx->G.px ? 3 : 1, iy = ctx->G.py ? 3 : 1, iz = ctx->G.pz ? 3 : 1;
-  k_sphere_mask<<<nsph * ix * iy * iz, NT, 0, ctx->stream>>>(ctx->G, ctx->grid.dx, ctx->grid.dy, ctx->grid.dz, xs,
-                                                              ys, zs, ix, iy, iz, d, mask);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
-  CK(e);
+  k_sphere_mask<<<nsph, 256, 0, ctx->stream>>>(ctx->G, ctx->grid.dx, ctx->grid.dy, ctx->grid.dz, xs, ys, zs, ix, iy,
+                                               iz, d, mask);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(ctx->stream));
   return 0;
 }
 

@@ -13,8 +13,9 @@
 //                           taps are 27 k16 steps whose A rows are shifted
 //                           halo rows (ldmatrix gather).  dgrad uses the same
 //                           kernel with the taps flipped and W transposed.
-//  k_conv3_wgrad<CIN, COUT> dW[t] += sum_v g[v]^T in[v + t], one tap per CTA
-//                           over a range of tiles, warps split the voxels.
+//  k_conv3_wgrad<CIN, COUT> dW[t] += sum_v g[v]^T in[v + t], all taps of 16 input
+//                           channels per CTA over a range of tiles, warps split
+//                           the taps.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -191,86 +192,139 @@ __host__ __device__ constexpr int conv_fwd_smem() {
 }
 
 // --------------------------------------------------------------- wgrad -----
-// CTA (tap, slice of tiles); 8 warps take the 16 voxel rows (z, y) of a tile,
-// two each.  A = g^T (COUT x voxels), B = in shifted by the tap (voxels x 16
-// input channels), both staged in shared memory and read with ldmatrix.trans.
+// dW[tap] += g^T (COUT x voxels) . in shifted by the tap (voxels x CIN), FP32.
+// A CTA takes 16 input channels (blockIdx.y), a group of taps (blockIdx.z) and a
+// run of tiles.  Per tile it stages the 256 voxels of g and the 720 halo voxels of
+// the input once for all its taps: each warp owns WTAPS taps whole, so a g fragment
+// serves them all, a tap is a shifted ldmatrix row, and no sums cross warps.  The
+// next tile's copies (cp.async) are in flight while a tile is computed.  A plane's
+// sums start from zero and are added to the CTA's in FP32: the tensor unit's
+// accumulation loses a little at every step, and chains of whole tile runs gave
+// up to ten times the error.
+// One tap a CTA, as before, read g and the input 27 times over: 1435 us for 48 -> 16
+// and 429 us for 16 -> 16 on four 64^3 volumes, against 153 and 65 us.
+template <int COUT>
+__host__ __device__ constexpr int wgrad_taps() {  // taps of a warp: its sums take 64 registers
+  return 64 / COUT;
+}
+template <int COUT>
+__host__ __device__ constexpr int wgrad_stage() {  // bytes of one tile's g and input
+  return 256 * (COUT * 2 + 16) + HVOX * RSB;
+}
+
+// 16 bytes global to shared, zeros when !full
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool full) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(full ? 16 : 0)
+               : "memory");
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(256) k_conv3_wgrad(const WgradArgs a) {
   constexpr int GRS = COUT * 2 + 16;  // shared bytes per voxel row of g
   constexpr int MT = COUT / 16;       // m tiles (output channels)
+  constexpr int NTAP = wgrad_taps<COUT>();
+  constexpr int STAGE = wgrad_stage<COUT>();
   extern __shared__ __align__(16) unsigned char smem[];
-  unsigned char *s_g = smem;                             // 256 rows of GRS
-  unsigned char *s_x = smem + 256 * GRS;                 // 256 rows of RSB (16 channels)
-  float *s_red = reinterpret_cast<float *>(smem + 256 * GRS + 256 * RSB);  // 8 warps x COUT x 16
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tap = blockIdx.y;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+  const int c0 = 16 * blockIdx.y, tap0 = 8 * NTAP * blockIdx.z + warp;  // taps tap0 + 8 i
   const int tx_n = (a.nx + CTX - 1) / CTX, ty_n = (a.ny + CTY - 1) / CTY, tz_n = (a.nz + CTZ - 1) / CTZ;
-  const long long ntiles = (long long)tx_n * ty_n * tz_n * a.nb;
+  const int ntiles = tx_n * ty_n * tz_n * a.nb;
   const long long vol = (long long)a.nx * a.ny * a.nz;
-  for (int c0 = 0; c0 < CIN; c0 += 16) {
-    float acc[MT][2][4];
+  const int t_begin = blockIdx.x * a.tiles_per_cta, t_end = min(t_begin + a.tiles_per_cta, ntiles);
+
+  auto stage = [&](int tile, int slot) {  // g (zero outside the volume) and the halo of the input
+    unsigned char *s_g = smem + slot * STAGE, *s_x = s_g + 256 * GRS;
+    int tt = tile;
+    const int bx = tt % tx_n * CTX;
+    tt /= tx_n;
+    const int by = tt % ty_n * CTY;
+    tt /= ty_n;
+    const int bz = tt % tz_n * CTZ;
+    const long long vb = (long long)(tt / tz_n) * vol;
+    {
+      const int lx = tid % CTX, ly = (tid / CTX) % CTY, lz = tid / (CTX * CTY);
+      const int ox = bx + lx, oy = by + ly, oz = bz + lz;
+      const bool inside = ox < a.nx && oy < a.ny && oz < a.nz;
+      const bf16 *src = a.g + a.cg_off + (inside ? (vb + ((long long)oz * a.ny + oy) * a.nx + ox) * a.ldg : 0);
+#pragma unroll
+      for (int q = 0; q < COUT / 8; q++) cp16(s_g + tid * GRS + q * 16, src + q * 8, inside);
+    }
+    for (int v = tid; v < HVOX; v += 256) {
+      int gx = bx + v % HTX - 1, gy = by + (v / HTX) % HTY - 1, gz = bz + v / (HTX * HTY) - 1;
+      const bool in = pad_axis(gx, a.nx, a.px) && pad_axis(gy, a.ny, a.py) && pad_axis(gz, a.nz, a.pz);
+      const bf16 *src = a.in + a.ci_off + c0 + (in ? (vb + ((long long)gz * a.ny + gy) * a.nx + gx) * a.ldi : 0);
+      cp16(s_x + v * RSB, src, in);
+      cp16(s_x + v * RSB + 16, src + 8, in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float acc[NTAP][MT][2][4], sum[NTAP][MT][2][4];
+#pragma unroll
+  for (int i = 0; i < NTAP; i++)
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll
       for (int n = 0; n < 2; n++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) acc[m][n][q] = 0.f;
-    const long long t_begin = (long long)blockIdx.x * a.tiles_per_cta;
-    const long long t_end = t_begin + a.tiles_per_cta < ntiles ? t_begin + a.tiles_per_cta : ntiles;
-    for (long long tile = t_begin; tile < t_end; tile++) {
-      long long tt = tile;
-      const int bx = (int)(tt % tx_n);
-      tt /= tx_n;
-      const int by = (int)(tt % ty_n);
-      tt /= ty_n;
-      const int bz = (int)(tt % tz_n);
-      const int vb = (int)(tt / tz_n);
-      // stage g (zero outside the volume) and the shifted input
-      for (int idx = tid; idx < 256 * (COUT / 8 + 2); idx += 256) {
-        const int v = idx % 256, part = idx / 256;  // parts 0..COUT/8-1: g; then 2 parts of x
-        const int lx = v % CTX, ly = (v / CTX) % CTY, lz = v / (CTX * CTY);
-        const int ox = bx * CTX + lx, oy = by * CTY + ly, oz = bz * CTZ + lz;
-        const bool inside = ox < a.nx && oy < a.ny && oz < a.nz;
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (part < COUT / 8) {
-          if (inside)
-            val = *reinterpret_cast<const uint4 *>(a.g + ((long long)vb * vol + ((long long)oz * a.ny + oy) * a.nx + ox) *
-                                                            a.ldg + a.cg_off + part * 8);
-          *reinterpret_cast<uint4 *>(s_g + v * GRS + part * 16) = val;
-        } else {
-          const int half = part - COUT / 8;
-          int gx = ox + dx, gy = oy + dy, gz = oz + dz;
-          if (inside && pad_axis(gx, a.nx, a.px) && pad_axis(gy, a.ny, a.py) && pad_axis(gz, a.nz, a.pz))
-            val = *reinterpret_cast<const uint4 *>(a.in + ((long long)vb * vol + ((long long)gz * a.ny + gy) * a.nx + gx) *
-                                                             a.ldi + a.ci_off + c0 + half * 8);
-          *reinterpret_cast<uint4 *>(s_x + v * RSB + half * 16) = val;
-        }
-      }
-      __syncthreads();
+        for (int q = 0; q < 4; q++) acc[i][m][n][q] = sum[i][m][n][q] = 0.f;
+  int shift[NTAP];  // a tap's place in the halo; taps past the last repeat the first (not added)
 #pragma unroll
-      for (int rr = 0; rr < 2; rr++) {
-        const int row = warp + 8 * rr;  // voxel row (z, y) of the tile: voxels row*16 .. +15
-        // B: two n tiles (input channels 0-7, 8-15), k = 16 voxels of the row
-        uint32_t b00, b01, b10, b11;
-        {
-          const int mi = lane >> 3, i = lane & 7;
-          const int v = row * 16 + i + (mi & 1) * 8;
-          ldsm_x4_t(b00, b01, b10, b11, s_x + v * RSB + (mi >> 1) * 16);
-        }
+  for (int i = 0; i < NTAP; i++) {
+    const int tap = tap0 + 8 * i < 27 ? tap0 + 8 * i : 0;
+    shift[i] = (tap / 9 * HTY + (tap / 3) % 3) * HTX + tap % 3;
+  }
+  if (t_begin < t_end) stage(t_begin, 0);
+  for (int tile = t_begin; tile < t_end; tile++) {
+    const int slot = (tile - t_begin) & 1;
+    if (tile + 1 < t_end) {
+      stage(tile + 1, slot ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const unsigned char *s_g = smem + slot * STAGE, *s_x = s_g + 256 * GRS;
+    const int mi = lane >> 3, li = lane & 7;
+#pragma unroll 1
+    for (int lz = 0; lz < CTZ; lz++) {
+#pragma unroll 2
+    for (int row = lz * CTY; row < (lz + 1) * CTY; row++) {  // 16 voxels of a row (z, y) of the tile
+      uint32_t af[MT][4];
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+        ldsm_x4_t(af[m][0], af[m][1], af[m][2], af[m][3],
+                  s_g + (row * 16 + li + (mi >> 1) * 8) * GRS + (m * 16 + (mi & 1) * 8) * 2);
+      const int hv = (row / CTY * HTY + row % CTY) * HTX + li + (mi & 1) * 8;
+#pragma unroll
+      for (int i = 0; i < NTAP; i++) {
+        uint32_t b00, b01, b10, b11;  // input channels 0-7 and 8-15, k = 16 voxels
+        ldsm_x4_t(b00, b01, b10, b11, s_x + (hv + shift[i]) * RSB + (mi >> 1) * 16);
 #pragma unroll
         for (int m = 0; m < MT; m++) {
-          uint32_t af[4];
-          const int mi = lane >> 3, i = lane & 7;
-          const int v = row * 16 + i + (mi >> 1) * 8;
-          ldsm_x4_t(af[0], af[1], af[2], af[3], s_g + v * GRS + (m * 16 + (mi & 1) * 8) * 2);
-          mma16816(acc[m][0], af, b00, b01);
-          mma16816(acc[m][1], af, b10, b11);
+          mma16816(acc[i][m][0], af[m], b00, b01);
+          mma16816(acc[i][m][1], af[m], b10, b11);
         }
       }
-      __syncthreads();
     }
-    // reduce the 8 warps' partial sums in shared memory, then add to dW
+#pragma unroll
+    for (int i = 0; i < NTAP; i++)
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            sum[i][m][n][q] += acc[i][m][n][q];
+            acc[i][m][n][q] = 0.f;
+          }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < NTAP; i++) {
+    const int tap = tap0 + 8 * i;
+    if (tap >= 27) continue;
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll
@@ -279,23 +333,14 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(const WgradArgs a) {
         for (int q = 0; q < 4; q++) {
           const int co = m * 16 + (lane >> 2) + (q >> 1) * 8;
           const int ci = n * 8 + (lane & 3) * 2 + (q & 1);
-          s_red[(warp * COUT + co) * 16 + ci] = acc[m][n][q];
+          atomicAdd(&a.dW[((long long)tap * COUT + co) * CIN + c0 + ci], sum[i][m][n][q]);
         }
-    __syncthreads();
-    for (int e = tid; e < COUT * 16; e += 256) {
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; w++) s += s_red[w * COUT * 16 + e];
-      const int co = e / 16, ci = e % 16;
-      atomicAdd(&a.dW[((long long)tap * COUT + co) * CIN + c0 + ci], s);
-    }
-    __syncthreads();
   }
 }
 
 template <int CIN, int COUT>
 constexpr int conv_wgrad_smem() {
-  return 256 * (COUT * 2 + 16) + 256 * RSB + 8 * COUT * 16 * 4;
+  return 2 * wgrad_stage<COUT>();
 }
 
 }  // namespace bbnet

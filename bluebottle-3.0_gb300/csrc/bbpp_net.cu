@@ -320,10 +320,23 @@ cudaError_t conv_wgrad_t(WgradArgs a, cudaStream_t s) {
   }
   const long long ntiles = (long long)((a.nx + CTX - 1) / CTX) * ((a.ny + CTY - 1) / CTY) *
                            ((a.nz + CTZ - 1) / CTZ) * a.nb;
-  int ctas = (int)std::min<long long>(ntiles, 64);
+  if (ntiles >= (1ll << 31)) return cudaErrorInvalidValue;
+  // one wave: every CTA adds its sums to dW once, so more CTAs are more atomics
+  static int wave = 0;
+  if (!wave) {
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3_wgrad<CIN, COUT>, 256, smem);
+    wave = std::max(1, sms) * std::max(1, per_sm);
+  }
+  constexpr int chunks = CIN / 16, groups = (27 + 8 * wgrad_taps<COUT>() - 1) / (8 * wgrad_taps<COUT>());
+  // and more roundings: eight tiles a CTA at least, on small volumes
+  int ctas = (int)std::min<long long>(std::min<long long>(ntiles, std::max<long long>(ntiles / 8, 16)),
+                                      std::max(1, wave / (chunks * groups)));
   a.tiles_per_cta = (int)((ntiles + ctas - 1) / ctas);
   ctas = (int)((ntiles + a.tiles_per_cta - 1) / a.tiles_per_cta);
-  dim3 grid(ctas, 27);
+  dim3 grid(ctas, chunks, groups);
   k_conv3_wgrad<CIN, COUT><<<grid, 256, smem, s>>>(a);
   return cudaGetLastError();
 }
@@ -538,31 +551,38 @@ __global__ void k_up_bwd(const bf16 *__restrict__ dout, int ldo, int off, int C,
 }
 
 // g[v][c] (ld C) = dout[v][c] (ld C) * (out[v][off + c] > 0)   (ReLU backward)
-__global__ void k_gate(const bf16 *__restrict__ dout, const bf16 *__restrict__ out, int ldo, int off, int C,
-                       long long nvox, bf16 *__restrict__ g) {
-  const long long n = nvox * C;
-  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < n; e += (long long)gridDim.x * 256) {
-    const long long v = e / C;
-    const int c = (int)(e - v * C);
-    g[e] = __bfloat162float(out[v * ldo + off + c]) > 0.f ? dout[e] : __float2bfloat16_rn(0.f);
-  }
-}
-
-// db[c] += sum_v g[v][c]
-__global__ void k_bias_grad(const bf16 *__restrict__ g, int C, long long nvox, float *db) {
-  __shared__ float s[256];
-  for (int c = 0; c < C; c++) {
-    float a = 0.f;
-    for (long long v = blockIdx.x * 256LL + threadIdx.x; v < nvox; v += (long long)gridDim.x * 256)
-      a += __bfloat162float(g[v * C + c]);
-    s[threadIdx.x] = a;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-      if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-      __syncthreads();
+// g = dout where the layer's output is positive, else 0; db[c] += sum_v g[v][c].
+// Eight channels (16 bytes) a thread; a thread keeps its channels from voxel to
+// voxel, so the bias sums stay in registers.  One pass: the gate and the bias
+// gradient apart took 71 + 35 us for 16 channels of four 64^3 volumes.
+__global__ void __launch_bounds__(256) k_gate_bias(const bf16 *__restrict__ dout, const bf16 *__restrict__ out,
+                                                   int ldo, int off, int C, long long nvox, bf16 *__restrict__ g,
+                                                   float *db) {
+  __shared__ float s[256][9];
+  const int parts = C / 8, part = threadIdx.x % parts, per = 256 / parts;  // C = 16, 32 or 64
+  float a[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) a[q] = 0.f;
+  for (long long v = blockIdx.x * (long long)per + threadIdx.x / parts; v < nvox; v += (long long)gridDim.x * per) {
+    const uint4 du = *reinterpret_cast<const uint4 *>(dout + v * C + part * 8);
+    const uint4 ou = *reinterpret_cast<const uint4 *>(out + v * ldo + off + part * 8);
+    float d[8], o[8];
+    bf8_unpack(du, d);
+    bf8_unpack(ou, o);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      d[q] = o[q] > 0.f ? d[q] : 0.f;
+      a[q] += d[q];
     }
-    if (threadIdx.x == 0) atomicAdd(&db[c], s[0]);
-    __syncthreads();
+    *reinterpret_cast<uint4 *>(g + v * C + part * 8) = bf8_pack(d);
+  }
+#pragma unroll
+  for (int q = 0; q < 8; q++) s[threadIdx.x][q] = a[q];
+  __syncthreads();
+  if (threadIdx.x < (unsigned)C) {
+    float t = 0.f;
+    for (int i = threadIdx.x / 8; i < 256; i += parts) t += s[i][threadIdx.x % 8];
+    atomicAdd(&db[threadIdx.x], t);
   }
 }
 
@@ -1027,8 +1047,7 @@ static int backward(bbpp_net *n, int nx, int ny, int nz, int nb) {
   k_head_bwd<<<nblocks(V), 256, 0, s>>>(n->dOUT, n->D1, n->w + n->head_w, V, n->dD1, G32 + n->head_w,
                                         G32 + n->head_b);
   // D1 = relu(conv(CAT1))
-  k_gate<<<nblocks(V * 16), 256, 0, s>>>(n->dD1, n->D1, 16, 0, 16, V, n->G);
-  k_bias_grad<<<nblocks(V) / 8 + 1, 256, 0, s>>>(n->G, 16, V, G32 + L[4].boff);
+  k_gate_bias<<<std::min(nblocks(V * 2), 1216), 256, 0, s>>>(n->dD1, n->D1, 16, 0, 16, V, n->G, G32 + L[4].boff);
   e = conv_wgrad(48, 16, wargs(nx, ny, nz, nb, n->CAT1, 48, 0, n->G, 16, G32 + L[4].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(16, 48, cargs(n, nx, ny, nz, nb, n->G, 16, 0, n->wt16 + L[4].woff, nullptr, n->dCAT1, 48, 0, 0), s);
@@ -1036,8 +1055,7 @@ static int backward(bbpp_net *n, int nx, int ny, int nz, int nb) {
   // CAT1[:, 0:32] = up(D2)
   k_up_bwd<<<nblocks(V2 * 32), 256, 0, s>>>(n->dCAT1, 48, 0, 32, nx, ny, nz, nb, n->dD2);
   // D2 = relu(conv(CAT2))
-  k_gate<<<nblocks(V2 * 32), 256, 0, s>>>(n->dD2, n->D2, 32, 0, 32, V2, n->G);
-  k_bias_grad<<<nblocks(V2) / 8 + 1, 256, 0, s>>>(n->G, 32, V2, G32 + L[3].boff);
+  k_gate_bias<<<std::min(nblocks(V2 * 4), 1216), 256, 0, s>>>(n->dD2, n->D2, 32, 0, 32, V2, n->G, G32 + L[3].boff);
   e = conv_wgrad(96, 32, wargs(hx, hy, hz, nb, n->CAT2, 96, 0, n->G, 32, G32 + L[3].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(32, 96, cargs(n, hx, hy, hz, nb, n->G, 32, 0, n->wt16 + L[3].woff, nullptr, n->dCAT2, 96, 0, 0), s);
@@ -1045,24 +1063,21 @@ static int backward(bbpp_net *n, int nx, int ny, int nz, int nb) {
   // CAT2[:, 0:64] = up(E3)
   k_up_bwd<<<nblocks(V4 * 64), 256, 0, s>>>(n->dCAT2, 96, 0, 64, hx, hy, hz, nb, n->dE3);
   // E3 = relu(conv(P2))
-  k_gate<<<nblocks(V4 * 64), 256, 0, s>>>(n->dE3, n->E3, 64, 0, 64, V4, n->G);
-  k_bias_grad<<<nblocks(V4) / 8 + 1, 256, 0, s>>>(n->G, 64, V4, G32 + L[2].boff);
+  k_gate_bias<<<std::min(nblocks(V4 * 8), 1216), 256, 0, s>>>(n->dE3, n->E3, 64, 0, 64, V4, n->G, G32 + L[2].boff);
   e = conv_wgrad(32, 64, wargs(qx, qy, qz, nb, n->P2, 32, 0, n->G, 64, G32 + L[2].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(64, 32, cargs(n, qx, qy, qz, nb, n->G, 64, 0, n->wt16 + L[2].woff, nullptr, n->dP2, 32, 0, 0), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   // E2 (in CAT2[:, 64:96]): skip gradient dCAT2[:, 64:96] + pool backward of dP2
   k_pool_bwd<<<nblocks(V2 * 32), 256, 0, s>>>(n->dP2, n->dCAT2, 96, 64, 32, hx, hy, hz, nb, n->dE2);
-  k_gate<<<nblocks(V2 * 32), 256, 0, s>>>(n->dE2, n->CAT2, 96, 64, 32, V2, n->G);
-  k_bias_grad<<<nblocks(V2) / 8 + 1, 256, 0, s>>>(n->G, 32, V2, G32 + L[1].boff);
+  k_gate_bias<<<std::min(nblocks(V2 * 4), 1216), 256, 0, s>>>(n->dE2, n->CAT2, 96, 64, 32, V2, n->G, G32 + L[1].boff);
   e = conv_wgrad(16, 32, wargs(hx, hy, hz, nb, n->P1, 16, 0, n->G, 32, G32 + L[1].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(32, 16, cargs(n, hx, hy, hz, nb, n->G, 32, 0, n->wt16 + L[1].woff, nullptr, n->dP1, 16, 0, 0), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   // E1 (in CAT1[:, 32:48]): skip gradient dCAT1[:, 32:48] + pool backward of dP1
   k_pool_bwd<<<nblocks(V * 16), 256, 0, s>>>(n->dP1, n->dCAT1, 48, 32, 16, nx, ny, nz, nb, n->dE1);
-  k_gate<<<nblocks(V * 16), 256, 0, s>>>(n->dE1, n->CAT1, 48, 32, 16, V, n->G);
-  k_bias_grad<<<nblocks(V) / 8 + 1, 256, 0, s>>>(n->G, 16, V, G32 + L[0].boff);
+  k_gate_bias<<<std::min(nblocks(V * 2), 1216), 256, 0, s>>>(n->dE1, n->CAT1, 48, 32, 16, V, n->G, G32 + L[0].boff);
   e = conv_wgrad(16, 16, wargs(nx, ny, nz, nb, n->X0, 16, 0, n->G, 16, G32 + L[0].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   NCK(cudaGetLastError());

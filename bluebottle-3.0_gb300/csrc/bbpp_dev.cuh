@@ -72,6 +72,7 @@ struct DevState {
   // number of steps; residual kernels write z = r / dL in place of r
   double pair[4];
   int pair_steps;
+  int pair_fresh;  // the pair (counted by fq) whose search direction is z, not p
   int zform;
 };
 

@@ -879,6 +879,17 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
   if (last_cta_reduce<3>(v, partials, st, nb, bid, s_red, tot) && tid == 0) resid_finish(st, tot, mode);
 }
 
+// A replaced residual that is not the one the recursion carried (FP32 lost it: a
+// solve that converges by more than 1e7 between two replacements) leaves a search
+// direction that is not conjugate to it, and CG never recovers from that: the
+// iterations stall or diverge.  They restart from the residual instead.  10% of
+// random solid cells at 160^3 to 1e-8: 5649 iterations without, under 100 with it.
+constexpr double kLostBeta = 4.0;
+// pairs: p is already formed when the residual comes; rz as the recursion had it
+__device__ __forceinline__ void pair_restart(DevState *st, double rz1, double rz) {
+  st->pair_fresh = (rz1 <= 1.5 * rz && rz <= 1.5 * rz1) ? -1 : st->fq;
+}
+
 // The device state after a residual: init (mode 0), replacement at a
 // checkpoint (1) or confirmation of a recursive convergence (2).  tot: (r,z),
 // (r,r), (rhs,rhs).
@@ -905,7 +916,9 @@ __device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3
     } else if (mode == 1) {
       st->replacements += 1;
       st->dlag = 0;  // x was settled before this residual
+      if (st->zform) pair_restart(st, rz1, st->rz * st->pair[1] * (st->pair_steps == 2 ? st->pair[3] : 1.0));
       finish_iteration(st, rz1, rr1, !st->zform);  // a pair's kernels have counted theirs
+      if (st->beta > kLostBeta) st->beta = 0.0;
       st->rr_ref = rr1;
       st->last_rep = st->iter;
     } else {  // confirm
@@ -920,7 +933,9 @@ __device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3
       } else if (isnan(rz1)) {
         st->done = DONE_NAN;
       } else {
+        if (st->zform) pair_restart(st, rz1, st->rz);
         st->beta = rz1 / st->rz;
+        if (st->beta > kLostBeta) st->beta = 0.0;
         st->rz = rz1;
         st->done = (st->iter > st->max_iter) ? DONE_MAX_ITER : RUNNING;
       }

@@ -203,6 +203,8 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   __shared__ int s_last;
   __shared__ int s_piece[2][8][3], s_np[4];
   if (*(volatile int *)&st->done) return;
+  // the first pair, and a restart after a replaced residual: p = z
+  const bool fresh = *(volatile int *)&st->pair_fresh == *(volatile int *)&st->fq - (STEP ? 1 : 0);
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
   const bool skip_one = *(volatile int *)&st->inject && blockIdx.x == 0 && blockIdx.y == 0;
@@ -300,7 +302,7 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
       return;
     }
     float *dst = which ? sz + (k % RING) * zrow : sp + (k % RING) * prow;
-    const float *src = (which ? zin : pin) + (size_t)plane * zp;
+    const float *src = (which || fresh ? zin : pin) + (size_t)plane * zp;
     for (int q = 0; q < s_np[which]; q++)
       bulk_load(dst + s_piece[which][q][0], src + s_piece[which][q][1], (unsigned int)s_piece[which][q][2], bar,
                 l2_policy(0));

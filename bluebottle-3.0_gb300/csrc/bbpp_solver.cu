@@ -996,7 +996,6 @@ int bbpp_pcg_loop_pair(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, flo
                        int *iters_out) {
   // a graph holds an even count of pairs, so that it starts on the same buffers
   const int per = (replace_every + 1) / 2, segments = per % 2 == 0 ? 1 : 2;
-  CK(cudaMemcpyAsync(p[0], z[0], sizeof(float) * (size_t)ctx->G.n, cudaMemcpyDeviceToDevice, ctx->stream));
   CK(cudaMemcpyAsync(hst, st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   long long rounds = 0;

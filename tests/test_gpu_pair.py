@@ -91,3 +91,23 @@ def test_pair_reports_wait_timeout_and_recovers(bbpp_lib, monkeypatch):
     assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
     x, rep = s.solve_host(b, mask, tol=1e-8, precision=bbpp.FP32_IR)
     assert rep.status == bbpp.CONVERGED and rep.true_rel <= 1e-8 * 1.01
+
+
+@pytest.mark.parametrize("dims,bc", [((40, 33, 37), "nnn"), ((24, 31, 40), "ppn"), ((33, 33, 33), "nnn"),
+                                     ((160, 160, 160), "ppp")])
+@pytest.mark.parametrize("resident", ["0", "1"])
+def test_lost_residual(bbpp_lib, monkeypatch, dims, bc, resident):
+    """So many solid cells that FP32 gains more than seven digits between two
+    replacements: the replaced residual is far from the recursion's, and the
+    iterations restart from it.  A restart reduces the residual by the six digits
+    that FP32 holds at least, so 1e-8 takes two of them: three times the FP64
+    iterations, and what is left to the next checkpoint each time."""
+    monkeypatch.setenv("BBPP_PERSIST", resident)
+    g, mask, b = problem(dims, bc, 5, 0.1, False)
+    ref = bbpp.Solver(g).solve_host(b, mask, tol=1e-8, precision=bbpp.FP64)
+    x, rep = bbpp.Solver(g).solve_host(b, mask, tol=1e-8, precision=bbpp.FP32_IR)
+    assert rep.status == bbpp.CONVERGED and rep.true_rel <= 1.01e-8
+    assert rep.iters <= 3 * ref[1].iters + 3 * 50
+    # the smallest eigenvalue of L / dL with a solid cell within a few cells of each
+    # fluid one is above 1e-2
+    assert np.abs(x - ref[0]).max() <= 1e2 * 2e-8 * np.linalg.norm(ref[0])

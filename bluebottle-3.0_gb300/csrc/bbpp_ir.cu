@@ -82,12 +82,12 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   hst->first = 1;
   // Pairs of iterations on grids of whole 16-byte rows (the mask is read in
   // words), the resident iteration on grids that fit the chip.  Where both apply
-  // the line is at 3.2M cells: 144^3 (3.0M) took 27.9 us an iteration resident and
-  // 26.9 in pairs, 200x144x106 with walls (3.1M) 30.5 and 31.8, 160^3 (4.1M) 32.2
-  // and 30.7, 128^3 (2.1M) 21 and 23.
+  // the line is at 4.2M cells, us an iteration of a solve, resident and in pairs:
+  // 128^3 (2.1M) 17.0 and 26.1, 144^3 (3.0M) 22.1 and 29.4, 160^3 (4.1M) 28.2 and
+  // 35.0 (walls 35.9 and 40.8), 168^3 (4.7M) 43.3 and 36.3, 176^3 (5.5M) 52.6 and 40.8.
   bool resident = bbpp_persist_ok(ctx, 4);
   const bool pair =
-      ctx->fused && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 && (!resident || n > 3200000);
+      ctx->fused && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 && (!resident || n > 4200000);
   if (pair) resident = false;
   hst->zform = pair ? 1 : 0;
   CK(cudaMemcpyAsync(st, hst, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));

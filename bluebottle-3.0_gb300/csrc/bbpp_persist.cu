@@ -4,11 +4,13 @@
 // One CTA per SM owns a box of cells and keeps the search direction of the box
 // and of its six faces' neighbours in shared memory from iteration to
 // iteration; r, Ap, x and the mask of the box stay there too as far as they
-// fit, and in L2 otherwise.  An iteration has two exchanges between the CTAs:
+// fit, and in L2 otherwise.  In FP64 an iteration has two exchanges between the CTAs:
 //   p = z + beta p on the box and its halo (the halo from the neighbours' z,
 //   published by the previous exchange, and the halo's own p); Ap = L p;
 //   exchange (p, Ap) -> alpha; r -= alpha Ap, x += alpha p, the z of the box's
 //   surface to global memory; exchange (r, z), (r, r) -> beta, stopping test.
+// In FP32 it has one (ONE below): all products of the iteration with (p, Ap), and
+// the neighbours' Ap instead of their z, from which the halo's r follows.
 // In an exchange every CTA stores its partial sums, counts itself in, and sums
 // all CTAs' slots in the same order, so all take the same decisions.  The
 // arithmetic per cell is that of k1_search2 and k2_update; the state at a
@@ -18,15 +20,15 @@
 //
 // Why: below ~3M cells the two-kernel iteration is bound by launches, by CTAs
 // that are too few and by the length of their z march.  An iteration here takes
-// two exchanges (2.5 us for (p, Ap), 4.5 us for (r, z) with its release of the
-// surface) plus, in FP64, the FP64 and integer pipes.  Measured, us per
-// iteration of a whole solve, two kernels against resident: FP64 32^3 44.7 ->
-// 10.8, 64^3 64 -> 17, 101x75x58 with walls 81 -> 22, 128^3 93 -> 58; FP32 128^3
-// 39 (fused kernel) -> 21, 200x144x106 69 -> 30.
+// its exchanges (2.5 us for (p, Ap), 4.5 us with the release of the surface) plus,
+// in FP64, the FP64 and integer pipes.  Measured, us per iteration of a whole
+// solve, kernel by kernel against resident: FP64 32^3 44.7 -> 10.8, 64^3 64 -> 16,
+// 101x75x58 with walls 81 -> 23, 128^3 93 -> 53; FP32 128^3 39 -> 17 (20 with two
+// exchanges), 200x144x106 with walls 69 -> 28 (31), 96^3 10.0 (13.2).
 //
 // A grid takes this path when p of its largest box fits a CTA's shared memory
-// (about 3M cells in FP64, 4M in FP32): up to there it was the faster one at
-// every size measured.
+// (about 3M cells in FP64, 6.8M in FP32); FP32 grids that can go in pairs do so
+// from 4.2M cells on.
 //
 // Every wait is bounded (one second of globaltimer, or the state's wait_ns): a
 // CTA whose wait runs out ends the solve with DONE_TIMEOUT and returns, and so
@@ -46,7 +48,7 @@ using namespace bbpp;
 namespace {
 
 constexpr int kMaxCtas = 256;          // one per SM
-constexpr int kSmemCap = 226 * 1024;   // static and dynamic shared memory of a CTA
+constexpr int kSmemCap = 227 * 1024;   // static and dynamic shared memory of a CTA
 
 struct __align__(16) Slot {
   double v;
@@ -61,17 +63,18 @@ struct bbpp_exchange {
   unsigned long long pad[14];
   unsigned long long arrived;     // CTAs that have put their slots, over all exchanges
   unsigned long long pad2[15];
-  Slot slot[3][kMaxCtas];         // (p, Ap); (r, z); (r, r)
+  Slot slot[2][7][kMaxCtas];      // by an exchange's parity and product
 };
 
 namespace {
 
 // The split of the grid into boxes, and what of a box lives in shared memory:
-// level 2: r, Ap, x and the mask; 1: r, Ap and the mask; 0: only p.
+// level 2: r, Ap, x and the mask; 1: r and Ap; 0: only p.
 struct Boxes {
   int sx, sy, sz, nb;
+  int one;                         // one exchange an iteration
   int level;
-  int off_r, off_a, off_x, off_m;  // byte offsets in dynamic shared memory
+  int off_r, off_a, off_x, off_m, off_h, off_c;  // byte offsets in dynamic shared memory
   int smem;                        // dynamic shared memory of a CTA
 };
 
@@ -209,6 +212,84 @@ __device__ __forceinline__ void exchange(const double (&v)[NV], double (&tot)[NV
   }
 }
 
+// The same for the NV products of a one-exchange iteration (NV <= 7), each summed by a
+// warp of its own: over the CTA's threads (FP32 partial sums as unevaluated pairs of
+// floats, 48 bits), then over the CTAs' slots, in fixed order.  Warp 7 counts the CTA
+// in, its earlier global writes before it, and waits.  Totals in s_tot.
+struct PairF {
+  float hi, lo;
+};
+__device__ __forceinline__ double sum_strided(const float *v, int n, int lane) {
+  PairF a = {v[lane], 0.f};
+  for (int e = lane + 32; e < n; e += 32) {  // two-sum (Knuth)
+    const float x = v[e], s = __fadd_rn(a.hi, x), b = __fsub_rn(s, a.hi);
+    a.lo = __fadd_rn(a.lo, __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    a.hi = s;
+  }
+  return widen_f32(a.hi) + widen_f32(a.lo);
+}
+template <int NV, int NTH>
+__device__ __forceinline__ void exchange_all(const float (&v)[NV], double *s_tot, bbpp_exchange *ex,
+                                             Slot (*slots)[kMaxCtas], int nb, unsigned long long n,
+                                             unsigned long long want, unsigned long long limit, bool silent,
+                                             float *s_part, int *s_bad) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double a = 0.0;
+#pragma unroll
+  for (int q0 = 0; q0 < NV; q0 += 4) {  // four at a time, for less shared memory
+    if (q0) __syncthreads();
+#pragma unroll
+    for (int q = q0; q < NV && q < q0 + 4; q++) s_part[(q - q0) * NTH + tid] = v[q];
+    __syncthreads();
+    if (warp >= q0 && warp < q0 + 4 && warp < NV) a = warp_sum(sum_strided(s_part + (warp - q0) * NTH, NTH, lane));
+  }
+  if (warp < NV) {
+    if (lane == 0 && !silent) slot_put(&slots[warp][blockIdx.x], a, n);
+  } else if (tid == 7 * 32) {
+    if (!silent) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      asm volatile("red.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(&ex->arrived) : "memory");
+    }
+    unsigned long long have, t0 = 0;
+    for (unsigned int k = 1;; k++) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(have) : "l"(&ex->arrived) : "memory");
+      if (have >= want) break;
+      if ((k & 255u) == 0) {  // a look at the clock now and then
+        const unsigned long long t = timer_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > limit) {
+          *s_bad = 1;
+          break;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < NV) {
+    const bool wait = *(volatile int *)s_bad == 0;
+    constexpr int K = kMaxCtas / 32;
+    double t[K];
+    bool got[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      t[k] = 0.0;
+      got[k] = lane + 32 * k < nb ? slot_get(&slots[warp][lane + 32 * k], n, t[k]) : true;
+    }
+    a = 0.0;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      // the arrivals may be seen before a slot: a few polls
+      for (unsigned int w = 0; !got[k] && wait && w < (1u << 20); w++)
+        got[k] = slot_get(&slots[warp][lane + 32 * k], n, t[k]);
+      if (!got[k]) *s_bad = 1;
+      if (32 * k < nb) a += t[k];
+    }
+    a = warp_sum(a);
+    if (lane == 0) s_tot[warp] = a;
+  }
+  __syncthreads();
+}
+
 }  // namespace
 
 // A thread owns columns of the box: with at most NTH columns, one column and
@@ -216,17 +297,26 @@ __device__ __forceinline__ void exchange(const double (&v)[NV], double (&tot)[NV
 // Along z the addresses advance by constants and the z neighbours of p are the
 // values just read.  Loads go out U cells at a time ahead of the stores (the
 // compiler cannot tell the box's arrays apart).
-template <typename T, int NTH, int LEVEL, bool MASK, bool ISO>
+//
+// ONE (FP32): one exchange an iteration.  (p,Ap) gives alpha; beta and the stopping
+// test come from (r,z) - 2 alpha (Ap,z) + alpha^2 (Ap,Ap/dL), and (r,r) alike without
+// dL, of products summed beside it.  The exact (r,z) of the next iteration restarts
+// the expansion, so no error accumulates (as in the fused kernel).  r, x and p
+// advance in one pass after it, the halo's r by the neighbours' Ap.  In FP64 the
+// three more products a cell cost as much as the exchange saves from 64^3 on.
+template <typename T, int NTH, int LEVEL, bool ONE, bool MASK, bool ISO>
 __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B, T *p0,
                                                     T *p1, T *__restrict__ rg, T *__restrict__ ag,
                                                     T *__restrict__ xg, const uint8_t *__restrict__ mask,
                                                     DevState *st, bbpp_exchange *ex, int replace_every) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ T s_inv[27], s_im1[27], s_dm1[27];  // per class 1/dL, 1/dL - 1, dL - 1
-  __shared__ double s_part[2 * NTH];
+  __shared__ __align__(16) unsigned char s_raw[ONE ? 4 * NTH * sizeof(T) : 2 * NTH * sizeof(double)];
+  double *const s_part = reinterpret_cast<double *>(s_raw);
   __shared__ double s_w[2][8];
+  __shared__ double s_tot[8];
   __shared__ double s_alpha, s_beta;
-  __shared__ int s_bad, s_done;
+  __shared__ int s_bad, s_done, s_exact;
   constexpr int U = sizeof(T) == 8 ? 2 : 4;
   if (*(volatile int *)&st->done) return;
   unsigned long long epoch = *(volatile unsigned long long *)&ex->epoch;
@@ -248,6 +338,7 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
     s_beta = first ? 0.0 : *(volatile double *)&st->beta;
     s_bad = 0;
     s_done = RUNNING;
+    s_exact = 0;
   }
   // thread 0's copy of the solve's scalars
   double rz = *(volatile double *)&st->rz, rz_last = *(volatile double *)&st->rz_last,
@@ -288,6 +379,11 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
   // between a launch's entry and exit p0 is free: it carries the z of the boxes'
   // surfaces to their neighbours
   T *const zg = p0;
+  T *const sh = reinterpret_cast<T *>(smem_raw + B.off_h);  // ONE: r of the halo
+  uint8_t *const sc = smem_raw + B.off_c;                   // ONE: its class
+  // the halo has cells at a wall
+  const bool near_wall = (!G.px && (x0 <= 1 || x0 + bx >= nx - 1)) || (!G.py && (y0 <= 1 || y0 + by >= ny - 1)) ||
+                         (!G.pz && (z0 <= 1 || z0 + bz >= nz - 1));
   T *const sp = reinterpret_cast<T *>(smem_raw);
   T *const rs = reinterpret_cast<T *>(smem_raw + B.off_r);
   T *const as = reinterpret_cast<T *>(smem_raw + B.off_a);
@@ -392,7 +488,7 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
         if (LEVEL >= 1) rs[e] = rg[g];
         if (LEVEL >= 2) xs[e] = lag ? fma(alpha, p, xg[g]) : xg[g];
         else if (lag) xg[g] = fma(alpha, p, xg[g]);
-        if (MASK && LEVEL >= 1) ms[e] = mask[g];
+        if (MASK && LEVEL >= 2) ms[e] = mask[g];
       }
     }
     for (int h = tid; h < halo; h += NTH) {
@@ -400,6 +496,7 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
       unsigned int g;
       const bool in = halo_cell(h, o, g, cls, std::false_type());
       sp[o] = in && !first ? po[g] : T(0);
+      if (ONE && near_wall) sc[h] = 0;
     }
   }
   __syncthreads();
@@ -415,7 +512,14 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
         int o, cls;
         unsigned int g;
         if (!halo_cell(h, o, g, cls, std::true_type())) continue;
-        T z = rg[g];
+        const T r = rg[g];
+        if (ONE) {
+          sh[h] = r;
+          if (near_wall) sc[h] = (uint8_t)cls;
+          sp[o] = fma(s_im1[cls], r, first ? r : fma(beta, sp[o], r));
+          continue;
+        }
+        T z = r;
         if (cls) z *= s_inv[cls];
         sp[o] = first ? z : fma(beta, sp[o], z);
       }
@@ -481,7 +585,7 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
           w[k] = qk[-1];
           n[k] = qk[PW];
           s[k] = qk[-PW];
-          solid[k] = MASK && (LEVEL >= 1 ? ms[c.e + ncol * (z + kk)]
+          solid[k] = MASK && (LEVEL >= 2 ? ms[c.e + ncol * (z + kk)]
                                          : __ldg(mask + c.g + plane * (unsigned int)(z + kk))) != 0;
         }
 #pragma unroll
@@ -557,55 +661,324 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
     v[0] = (double)rr + (double)corr;
     v[1] = (double)rr;
   };
-
-  bool checkpoint = false;
-  for (;;) {
-    it++;
-    checkpoint = it % replace_every == 0;
-    direction();
-    first = false;
-    __syncthreads();
-    {
-      const double v[1] = {stencil()};
-      double tot[1];
-      ++epoch;
-      want += (unsigned long long)B.nb;
-      exchange<1, NTH>(v, tot, ex, ex->slot, B.nb, epoch, want, limit, false, silent0 && it == it0 + 1, s_part, s_w, &s_bad);
-      if (tid == 0 && !s_bad) {
-        pap = tot[0];
-        const double a = rz / pap;
-        s_alpha = a;
-        trace_put(trace_a, trace_n, it - 1, a);
-      }
-    }
-    __syncthreads();
-    if (s_bad || checkpoint) break;
-    {
-      double v[2], tot[2];
-      update(v);
-      ++epoch;
-      want += (unsigned long long)B.nb;
-      exchange<2, NTH>(v, tot, ex, ex->slot + 1, B.nb, epoch, want, limit, true, false, s_part, s_w, &s_bad);
-      if (tid == 0 && !s_bad) {
-        // finish_iteration on the local scalars
-        const double rz1 = tot[0], rr1 = tot[1];
-        rz_last = rz1;
-        rr_last = rr1;
-        const bool conv = (stop == 0 ? rz1 : rr1) <= tol2bb;
-        if (conv) {
-          s_done = it > max_iter ? DONE_MAX_ITER : (stop == 0 ? DONE_CONVERGED : DONE_PENDING);
-        } else if (isnan(rz1)) {
-          s_done = DONE_NAN;
-        } else {
-          s_beta = rz1 / rz;
-          trace_put(trace_b, trace_n, it - 1, s_beta);
-          rz = rz1;
-          if (it > max_iter) s_done = DONE_MAX_ITER;
+  // ONE: Ap = L p with its products, Ap of the box's surface to wg; v: (p,Ap),
+  // (r,r), (r,Ap), (Ap,Ap) and, of the last three with 1/dL, what the walls add
+  auto stencil_all = [&](T *wg, T (&v)[7]) {
+#pragma unroll
+    for (int k = 0; k < 7; k++) v[k] = T(0);
+    for (int col = col0; col < ncol; col += NTH) {
+      const Col c = column(col);
+      const bool side = c.lx == 0 || c.lx == bx - 1 || c.ly == 0 || c.ly == by - 1;
+      const T *q = sp + c.o + PP * za;
+      T pb = za < zb ? q[-PP] : T(0), pc = za < zb ? q[0] : T(0);
+      for (int z = za; z < zb; z += U) {
+        T t[U], e[U], w[U], n[U], s[U], a[U], cc[U], r[U];
+        bool solid[U];
+        const T *qz = sp + c.o + PP * z;
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          const int kk = min(k, zb - 1 - z);
+          const T *qk = qz + PP * kk;
+          t[k] = qk[PP];
+          e[k] = qk[1];
+          w[k] = qk[-1];
+          n[k] = qk[PW];
+          s[k] = qk[-PW];
+          r[k] = LEVEL >= 1 ? rs[c.e + ncol * (z + kk)] : rg[c.g + plane * (unsigned int)(z + kk)];
+          solid[k] = MASK && (LEVEL >= 2 ? ms[c.e + ncol * (z + kk)]
+                                         : __ldg(mask + c.g + plane * (unsigned int)(z + kk))) != 0;
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          cc[k] = pc;
+          a[k] = apply_box<T, ISO>(G, pc, e[k], w[k], n[k], s[k], t[k], pb, solid[k]);
+          if (solid[k]) a[k] = T(0);
+          pb = pc;
+          pc = t[k];
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          if (z + k >= zb) break;
+          const unsigned int g = c.g + plane * (unsigned int)(z + k);
+          if (LEVEL >= 1) as[c.e + ncol * (z + k)] = a[k];
+          else ag[g] = a[k];
+          if (side || z + k == 0 || z + k == bz - 1) wg[g] = a[k];
+          v[0] = fma(cc[k], a[k], v[0]);
+          v[1] = fma(r[k], r[k], v[1]);
+          v[2] = fma(r[k], a[k], v[2]);
+          v[3] = fma(a[k], a[k], v[3]);
         }
       }
     }
+    if (wf) {
+      __syncthreads();
+      wall_cells([&](int e, int o, unsigned int g, int cls) {
+        T *ap = LEVEL >= 1 ? as + e : ag + g;
+        const T p = sp[o], q = s_dm1[cls] * p, a0 = *ap, a = a0 + q, r = LEVEL >= 1 ? rs[e] : rg[g];
+        const T im = s_im1[cls];
+        *ap = a;
+        wg[g] = a;
+        v[0] = fma(p, q, v[0]);
+        v[2] = fma(r, q, v[2]);
+        v[3] = fma(q, a + a0, v[3]);
+        v[4] = fma(im * r, r, v[4]);
+        v[5] = fma(im * r, a, v[5]);
+        v[6] = fma(im * a, a, v[6]);
+      });
+    }
+  };
+  // ONE: r -= alpha Ap and p = z + beta p on the halo, with the roundings of the
+  // boxes that own its cells
+  auto turn_halo = [&](const T *wg) {
+    const T alpha = (T)s_alpha, beta = (T)s_beta;
+    constexpr int H = 6;
+    for (int h0 = tid; h0 < halo; h0 += H * NTH) {
+      T w[H];
+      int o[H];
+#pragma unroll
+      for (int k = 0; k < H; k++) {
+        if (h0 + k * NTH >= halo) break;
+        unsigned int g;
+        int cls;
+        if (!halo_cell(h0 + k * NTH, o[k], g, cls, std::false_type())) o[k] = -1;
+        w[k] = o[k] >= 0 ? __ldcg(wg + g) : T(0);
+      }
+#pragma unroll
+      for (int k = 0; k < H; k++) {
+        if (h0 + k * NTH >= halo) break;
+        if (o[k] < 0) continue;
+        const T r = fma(-alpha, w[k], sh[h0 + k * NTH]);
+        sh[h0 + k * NTH] = r;
+        sp[o[k]] = fma(beta, sp[o[k]], r);
+      }
+    }
+    if (!near_wall) return;
+#pragma unroll 1
+    for (int h = tid; h < halo; h += NTH) {
+      if (sc[h] == 0) continue;
+      int o, cls;
+      unsigned int g;
+      halo_cell(h, o, g, cls, std::false_type());
+      sp[o] = fma(s_im1[sc[h]], sh[h], sp[o]);
+    }
+  };
+  // ONE: what 1 / dL adds to p at the walls
+  auto turn_walls = [&]() {
+    if (!wf) return;
     __syncthreads();
-    if (s_bad || s_done != RUNNING) break;
+    wall_cells([&](int e, int o, unsigned int g, int cls) {
+      sp[o] = fma(s_im1[cls], LEVEL >= 1 ? rs[e] : rg[g], sp[o]);
+    });
+  };
+  // ONE: r -= alpha Ap, x += alpha p and, with `next`, the next p on the box and its halo
+  auto advance = [&](const T *wg, bool next) {
+    const T alpha = (T)s_alpha, beta = (T)s_beta;
+    if (next) turn_halo(wg);
+    for (int col = col0; col < ncol; col += NTH) {
+      const Col c = column(col);
+      for (int z = za; z < zb; z += U) {
+        T r[U], a[U], x[U], p[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          const int zz = min(z + k, zb - 1), e = c.e + ncol * zz;
+          const unsigned int g = c.g + plane * (unsigned int)zz;
+          x[k] = LEVEL >= 2 ? xs[e] : xg[g];
+          r[k] = LEVEL >= 1 ? rs[e] : rg[g];
+          a[k] = LEVEL >= 1 ? as[e] : ag[g];
+          p[k] = sp[c.o + PP * zz];
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          if (z + k >= zb) break;
+          const int e = c.e + ncol * (z + k);
+          const unsigned int g = c.g + plane * (unsigned int)(z + k);
+          const T rn = fma(-alpha, a[k], r[k]);
+          const T xn = fma(alpha, p[k], x[k]);
+          if (LEVEL >= 2) xs[e] = xn;
+          else xg[g] = xn;
+          if (LEVEL >= 1) rs[e] = rn;
+          else rg[g] = rn;
+          if (next) sp[c.o + PP * (z + k)] = fma(beta, p[k], rn);
+        }
+      }
+    }
+    if (next) turn_walls();
+  };
+
+  bool checkpoint = false;
+  if constexpr (ONE) {
+    const bool walls = !(G.px && G.py && G.pz);
+    // an exchange of NV sums into s_tot
+    auto meet = [&](auto &v, bool silent) {
+      constexpr int NV = sizeof(v) / sizeof(float);
+      ++epoch;
+      want += (unsigned long long)B.nb;
+      exchange_all<NV, NTH>(v, s_tot, ex, ex->slot[epoch & 1], B.nb, epoch, want, limit, silent,
+                            reinterpret_cast<float *>(s_raw), &s_bad);
+    };
+    // finish_iteration on thread 0's scalars
+    auto finish = [&](double rz1, double rr1) {
+      rz_last = rz1;
+      rr_last = rr1;
+      const bool conv = (stop == 0 ? rz1 : rr1) <= tol2bb;
+      if (conv) {
+        s_done = it > max_iter ? DONE_MAX_ITER : (stop == 0 ? DONE_CONVERGED : DONE_PENDING);
+      } else if (isnan(rz1)) {
+        s_done = DONE_NAN;
+      } else {
+        s_beta = rz1 / rz;
+        trace_put(trace_b, trace_n, it - 1, s_beta);
+        rz = rz1;
+        if (it > max_iter) s_done = DONE_MAX_ITER;
+      }
+    };
+    T v[7];
+    auto meet_all = [&](bool silent) {
+      if (walls) {
+        meet(v, silent);
+      } else {
+        T u[4] = {v[0], v[1], v[2], v[3]};
+        meet(u, silent);
+      }
+    };
+    it++;
+    direction();
+    first = false;
+    for (;;) {
+      for (;; it++) {
+        checkpoint = it % replace_every == 0;
+        __syncthreads();
+        // by the iteration's parity, as p is stored at the end: a slow neighbour may
+        // still read the other buffer, which carries the iteration before's
+        T *const wg = (it & 1) ? p1 : p0;
+        stencil_all(wg, v);
+        meet_all(silent0 && it == it0 + 1);
+        if (tid == 0 && !s_bad) {
+          const double wr = walls ? s_tot[4] : 0.0, wa = walls ? s_tot[5] : 0.0, waa = walls ? s_tot[6] : 0.0;
+          const double rr = s_tot[1];
+          rz = rr + wr;
+          pap = s_tot[0];
+          const double al = rz / pap;
+          s_alpha = al;
+          trace_put(trace_a, trace_n, it - 1, al);
+          const double rz1 = rz - 2.0 * al * (s_tot[2] + wa) + al * al * (s_tot[3] + waa);
+          const double rr1 = rr - 2.0 * al * s_tot[2] + al * al * s_tot[3];
+          // what a step leaves of the residual is known to some 1e-7 of what was
+          // there; where that is not enough (or is NaN), from the residual itself
+          if (!checkpoint) {
+            if (rz1 >= 0.03 * rz && rr1 >= 0.03 * rr) finish(rz1, rr1);
+            else s_exact = 1;
+          }
+        }
+        __syncthreads();
+        if (s_bad || checkpoint || s_exact) break;
+        const bool next = s_done == RUNNING;
+        advance(wg, next);
+        if (!next) break;
+      }
+      if (s_bad || !s_exact) break;
+      // the step, the sums of the residual it leaves and the next p one by one
+      const T alpha = (T)s_alpha;
+      for (int k = 0; k < 7; k++) v[k] = T(0);
+#pragma unroll 1
+      for (int col = col0; col < ncol; col += NTH) {
+        const Col c = column(col);
+#pragma unroll 1
+        for (int z = za; z < zb; z++) {
+          const int e = c.e + ncol * z;
+          const unsigned int g = c.g + plane * (unsigned int)z;
+          T &r = LEVEL >= 1 ? rs[e] : rg[g], &x = LEVEL >= 2 ? xs[e] : xg[g];
+          r = fma(-alpha, LEVEL >= 1 ? as[e] : ag[g], r);
+          x = fma(alpha, sp[c.o + PP * z], x);
+          v[1] = fma(r, r, v[1]);
+        }
+      }
+      __syncthreads();
+      if (wf)
+        wall_cells([&](int e, int, unsigned int g, int cls) {
+          const T r = LEVEL >= 1 ? rs[e] : rg[g];
+          v[4] = fma(s_im1[cls] * r, r, v[4]);
+        });
+      meet_all(false);
+      if (tid == 0) {
+        s_exact = 0;
+        if (!s_bad) finish(s_tot[1] + (walls ? s_tot[4] : 0.0), s_tot[1]);
+      }
+      __syncthreads();
+      if (s_bad || s_done != RUNNING) break;
+      const T beta = (T)s_beta;
+      const T *const wg = (it & 1) ? p1 : p0;
+#pragma unroll 1
+      for (int h = tid; h < halo; h += NTH) {
+        int o, cls;
+        unsigned int g;
+        if (!halo_cell(h, o, g, cls, std::true_type())) continue;
+        const T r = fma(-alpha, __ldcg(wg + g), sh[h]);
+        sh[h] = r;
+        sp[o] = fma(s_im1[cls], r, fma(beta, sp[o], r));
+      }
+#pragma unroll 1
+      for (int col = col0; col < ncol; col += NTH) {
+        const Col c = column(col);
+#pragma unroll 1
+        for (int z = za; z < zb; z++) {
+          T &p = sp[c.o + PP * z];
+          p = fma(beta, p, LEVEL >= 1 ? rs[c.e + ncol * z] : rg[c.g + plane * (unsigned int)z]);
+        }
+      }
+      turn_walls();
+      it++;
+    }
+    __syncthreads();
+  } else {
+    for (;;) {
+      it++;
+      checkpoint = it % replace_every == 0;
+      direction();
+      first = false;
+      __syncthreads();
+      {
+        const double v[1] = {stencil()};
+        double tot[1];
+        ++epoch;
+        want += (unsigned long long)B.nb;
+        exchange<1, NTH>(v, tot, ex, ex->slot[0], B.nb, epoch, want, limit, false, silent0 && it == it0 + 1, s_part, s_w, &s_bad);
+        if (tid == 0 && !s_bad) {
+          pap = tot[0];
+          const double a = rz / pap;
+          s_alpha = a;
+          trace_put(trace_a, trace_n, it - 1, a);
+        }
+      }
+      __syncthreads();
+      if (s_bad || checkpoint) break;
+      {
+        double v[2], tot[2];
+        update(v);
+        ++epoch;
+        want += (unsigned long long)B.nb;
+        exchange<2, NTH>(v, tot, ex, ex->slot[0] + 1, B.nb, epoch, want, limit, true, false, s_part, s_w, &s_bad);
+        if (tid == 0 && !s_bad) {
+          // finish_iteration on the local scalars
+          const double rz1 = tot[0], rr1 = tot[1];
+          rz_last = rz1;
+          rr_last = rr1;
+          const bool conv = (stop == 0 ? rz1 : rr1) <= tol2bb;
+          if (conv) {
+            s_done = it > max_iter ? DONE_MAX_ITER : (stop == 0 ? DONE_CONVERGED : DONE_PENDING);
+          } else if (isnan(rz1)) {
+            s_done = DONE_NAN;
+          } else {
+            s_beta = rz1 / rz;
+            trace_put(trace_b, trace_n, it - 1, s_beta);
+            rz = rz1;
+            if (it > max_iter) s_done = DONE_MAX_ITER;
+          }
+        }
+      }
+      __syncthreads();
+      if (s_bad || s_done != RUNNING) break;
+    }
   }
 
   if (!s_bad) {
@@ -658,21 +1031,26 @@ struct bbpp_persist_state {
 
 namespace {
 
-constexpr size_t static_smem(int nth) { return 16 * (size_t)nth + 2048; }
+constexpr size_t static_smem(int nth) { return 16 * (size_t)nth + 1024; }
 
 // The split into at most `most` boxes that costs a thread least: the cells of
 // its columns (see k_persist), and the halo cells at half a cell's cost (the x
 // faces, whose cells lie in a sector each, at a cell's).  p of a box
 // with its halo must fit `cap` bytes.
-bool plan_boxes(const GeoL &G, int most, int elem, int nth, Boxes *out) {
+bool plan_boxes(const GeoL &G, int most, int elem, int nth, bool one, Boxes *out) {
   const size_t cap = kSmemCap - static_smem(nth);
+  const bool walls = !(G.px && G.py && G.pz);
+  // p of a box with its halo, and with one exchange the halo's r beside it
+  auto fixed = [&](size_t bx, size_t by, size_t bz) {
+    return (bx + 2) * (by + 2) * (bz + 2) * elem + (one ? 2 * (bx * by + bx * bz + by * bz) * (elem + walls) + 48 : 0);
+  };
   double best = 1e300;
   for (int sx = 1; sx <= G.nx && sx <= most; sx++)
     for (int sy = 1; sy <= G.ny && sx * sy <= most; sy++) {
       const int sz0 = std::min(G.nz, most / (sx * sy));
       const int bz = (G.nz + sz0 - 1) / sz0, sz = (G.nz + bz - 1) / bz;
       const int bx = (G.nx + sx - 1) / sx, by = (G.ny + sy - 1) / sy;
-      if ((size_t)(bx + 2) * (by + 2) * (bz + 2) * elem > cap) continue;
+      if (fixed(bx, by, bz) > cap) continue;
       const int ncol = bx * by, nseg = std::max(1, nth / ncol);
       const double steps = ncol <= nth ? (bz + nseg - 1) / nseg : (double)((ncol + nth - 1) / nth) * bz;
       const double cost = steps * nth + 1.0 * ((double)ncol + (double)bx * bz) + 2.0 * (double)by * bz;
@@ -685,16 +1063,21 @@ bool plan_boxes(const GeoL &G, int most, int elem, int nth, Boxes *out) {
     }
   if (best >= 1e300) return false;
   out->nb = out->sx * out->sy * out->sz;
+  out->one = one;
   const size_t bx = (G.nx + out->sx - 1) / out->sx, by = (G.ny + out->sy - 1) / out->sy,
                bz = (G.nz + out->sz - 1) / out->sz;
   auto up = [](size_t v) { return (v + 15) / 16 * 16; };
-  const size_t p = up((bx + 2) * (by + 2) * (bz + 2) * elem), one = up(bx * by * bz * elem), m = up(bx * by * bz);
+  const size_t p0 = up((bx + 2) * (by + 2) * (bz + 2) * elem), vec = up(bx * by * bz * elem), m = up(bx * by * bz);
+  out->off_h = (int)p0;
+  const size_t halo = 2 * (bx * by + bx * bz + by * bz);
+  out->off_c = (int)(p0 + up(halo * elem));
+  const size_t p = p0 + (one ? up(halo * elem) + (walls ? up(halo) : 0) : 0);
   out->off_r = (int)p;
-  out->off_a = (int)(p + one);
-  out->off_m = (int)(p + 2 * one);
-  out->off_x = (int)(p + 2 * one + m);
-  out->level = p + 3 * one + m <= cap ? 2 : (p + 2 * one + m <= cap ? 1 : 0);
-  out->smem = (int)(p + (out->level + (out->level > 0)) * one + (out->level > 0 ? m : 0));
+  out->off_a = (int)(p + vec);
+  out->off_x = (int)(p + 2 * vec);
+  out->off_m = (int)(p + 3 * vec);
+  out->level = p + 3 * vec + m <= cap ? 2 : (p + 2 * vec <= cap ? 1 : 0);
+  out->smem = (int)(p + (out->level + (out->level > 0)) * vec + (out->level == 2 ? m : 0));
   return true;
 }
 
@@ -706,17 +1089,22 @@ template <typename T> struct KernOf;
 template <> struct KernOf<double> { typedef Kern64 type; };
 template <> struct KernOf<float> { typedef Kern32 type; };
 
-template <typename T, int NTH, int LEVEL>
+template <typename T, int NTH, int LEVEL, bool ONE>
 typename KernOf<T>::type pick3(bool mask, bool iso) {
-  if (mask) return iso ? k_persist<T, NTH, LEVEL, true, true> : k_persist<T, NTH, LEVEL, true, false>;
-  return iso ? k_persist<T, NTH, LEVEL, false, true> : k_persist<T, NTH, LEVEL, false, false>;
+  if (mask) return iso ? k_persist<T, NTH, LEVEL, ONE, true, true> : k_persist<T, NTH, LEVEL, ONE, true, false>;
+  return iso ? k_persist<T, NTH, LEVEL, ONE, false, true> : k_persist<T, NTH, LEVEL, ONE, false, false>;
 }
-// small boxes (level 2 only) with 256 threads, the others with 512
-template <typename T>
-typename KernOf<T>::type pick(int nth, int level, bool mask, bool iso) {
-  if (nth == 256) return pick3<T, 256, 2>(mask, iso);
-  if (level == 2) return pick3<T, 512, 2>(mask, iso);
-  return level == 1 ? pick3<T, 512, 1>(mask, iso) : pick3<T, 512, 0>(mask, iso);
+// Small boxes (level 2 only) with 256 threads, the others with 512.
+Kern32 pick(float, int nth, const Boxes &B, bool mask, bool iso) {
+  if (!B.one) return pick3<float, 512, 0, false>(mask, iso);
+  if (nth == 256) return pick3<float, 256, 2, true>(mask, iso);
+  if (B.level == 2) return pick3<float, 512, 2, true>(mask, iso);
+  return B.level == 1 ? pick3<float, 512, 1, true>(mask, iso) : pick3<float, 512, 0, true>(mask, iso);
+}
+Kern64 pick(double, int nth, const Boxes &B, bool mask, bool iso) {
+  if (nth == 256) return pick3<double, 256, 2, false>(mask, iso);
+  if (B.level == 2) return pick3<double, 512, 2, false>(mask, iso);
+  return B.level == 1 ? pick3<double, 512, 1, false>(mask, iso) : pick3<double, 512, 0, false>(mask, iso);
 }
 
 }  // namespace
@@ -731,30 +1119,37 @@ void bbpp_persist_init(bbpp_ctx *ctx) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   if (!coop) return;
   const int most = std::min(ctx->sms, kMaxCtas);
-  for (int k = 0; k < 2; k++) {
+  // the warp-specialised fused kernel is asked for by its own variable
+  const char *ws = getenv("BBPP_FUSED_WS");
+  const int k0 = ws && atoi(ws) != 0 ? 1 : 0;
+  for (int k = k0; k < 2; k++) {
     const int elem = k ? 8 : 4;
     Boxes &B = t->box[k];
     t->nth[k] = (ctx->GL.n + most - 1) / most <= 512 ? 256 : 512;
-    bool ok = plan_boxes(ctx->GL, most, elem, t->nth[k], &B);
-    if (ok && t->nth[k] == 256 && B.level != 2) {
+    bool ok = plan_boxes(ctx->GL, most, elem, t->nth[k], k == 0, &B);
+    if (t->nth[k] == 256 && (!ok || B.level != 2)) {
       t->nth[k] = 512;
-      ok = plan_boxes(ctx->GL, most, elem, 512, &B);
+      ok = plan_boxes(ctx->GL, most, elem, 512, k == 0, &B);
     }
+    // FP32: one exchange an iteration where the halo's r fits beside p
+    if (!k && !ok) {
+      ok = plan_boxes(ctx->GL, most, elem, 512, false, &B);
+      B.level = 0;
+    }
+    const int all = kSmemCap - (int)static_smem(t->nth[k]);
     if (!ok) continue;
     // the attribute is a per-function cap shared by all contexts: the maximum,
     // set once per device (setting it and asking for the occupancy take ~1 ms)
     static std::atomic<unsigned int> ready[64];
-    const int variant = 4 * k + (t->nth[k] == 256 ? 3 : B.level);
+    const int variant = 8 * k + 4 * B.one + (t->nth[k] == 256 ? 3 : B.level);
     const bool known = dev < 64 && (ready[dev].load() >> variant & 1u);
     for (int v = 0; v < 4 && ok && !known; v++) {
-      const void *f = k ? (const void *)pick<double>(t->nth[k], B.level, v & 1, v & 2)
-                        : (const void *)pick<float>(t->nth[k], B.level, v & 1, v & 2);
-      ok = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSmemCap - (int)static_smem(t->nth[k])) == cudaSuccess;
+      const void *f = k ? (const void *)pick(0.0, t->nth[k], B, v & 1, v & 2)
+                        : (const void *)pick(0.f, t->nth[k], B, v & 1, v & 2);
+      ok = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, all) == cudaSuccess;
       int per_sm = 0;
       ok = ok &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, t->nth[k],
-                                                         (size_t)kSmemCap - static_smem(t->nth[k])) == cudaSuccess &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, t->nth[k], (size_t)all) == cudaSuccess &&
            per_sm >= 1;
     }
     cudaGetLastError();
@@ -809,7 +1204,7 @@ int bbpp_persist(bbpp_ctx *ctx, const uint8_t *mask, T *r, T *const p[2], T *Ap,
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const cudaError_t e =
-      cudaLaunchKernelEx(&cfg, pick<T>(ctx->persist->nth[k], B.level, mask != nullptr, ctx->GL.iso != 0), ctx->GL, B,
+      cudaLaunchKernelEx(&cfg, pick(T(0), ctx->persist->nth[k], B, mask != nullptr, ctx->GL.iso != 0), ctx->GL, B,
                          p[0], p[1], r, Ap, x, mask, st, ctx->persist->ex, replace_every);
   if (e != cudaSuccess) {
     bbpp_record_error(ctx, e, "k_persist", __LINE__);

@@ -26,7 +26,8 @@ def problem(dims, bc, seed, frac):
 
 # a box of one cell a direction, more columns than threads, walls on both sides of
 # a box, a periodic axis in one box, odd splits; the three levels of what lives
-# in shared memory in FP64 (about 0.9M and 1.15M cells) and FP32 (1.75M, 2.3M)
+# in shared memory in FP64 (about 0.9M and 1.15M cells) and FP32 (1.75M, 2.3M), and
+# FP32 boxes that leave no room for the halo's residual (two exchanges an iteration)
 CASES = [
     ((301, 2, 1), "ppp", 0.0, bbpp.FP64),
     ((1, 1, 7), "ppn", 0.0, bbpp.FP64),
@@ -38,6 +39,7 @@ CASES = [
     ((101, 90, 80), "nnp", 0.02, bbpp.FP32_IR),
     ((128, 125, 130), "ppn", 0.02, bbpp.FP32_IR),
     ((160, 150, 140), "pnn", 0.02, bbpp.FP32_IR),
+    ((183, 184, 184), "npp", 0.02, bbpp.FP32_IR),
 ]
 
 

@@ -202,7 +202,7 @@ __host__ __device__ constexpr int conv_fwd_smem() {
 // accumulation loses a little at every step, and chains of whole tile runs gave
 // up to ten times the error.
 // One tap a CTA, as before, read g and the input 27 times over: 1435 us for 48 -> 16
-// and 429 us for 16 -> 16 on four 64^3 volumes, against 153 and 65 us.
+// and 429 us for 16 -> 16 on four 64^3 volumes, against 189 and 70 us.
 template <int COUT>
 __host__ __device__ constexpr int wgrad_taps() {  // taps of a warp: its sums take 64 registers
   return 64 / COUT;

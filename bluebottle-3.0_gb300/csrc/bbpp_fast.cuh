@@ -15,8 +15,8 @@
 // Ap = 0 there.  A fluid cell's solid neighbour then contributes p = 0, which
 // is the reference's dropped off-diagonal (src/solver_kernel.cu:691-707).
 //
-//  k1_search2 p = invM r + beta p_old on a 64x8 tile plus halo (two cells per
-//             thread), ring of four planes in shared memory while the CTA
+//  k1_search2 p = invM r + beta p_old on a 64x8 or 64x16 tile plus halo (pairs of
+//             cells), ring of four planes in shared memory while the CTA
 //             marches in z; Ap = L p and the (p, Ap) partial.
 //  k2_update  r -= alpha Ap, (r,r) and the wall correction of (r,z), 16-byte
 //             vector loads; optionally in the reverse of the search kernel's
@@ -227,21 +227,22 @@ __device__ __forceinline__ double apply_L0<double, true>(const GeoL &G, double p
 // FP64 work on the next plane runs beside others' integer sums of this one); then Ap = L p_new and the (p, Ap) partial.
 // Replaces PP_update_search + exchange + PP_spmv_shared_load + thrust (p,Ap)
 // (src/solver_kernel.cu:528-713,906-927, src/cuda_solver.cu:201-205,256-263).
-// Two x-adjacent cells per thread: a tile is 64 x 8 cells (32 x 8 threads, one row each).  Halo rows are loaded as aligned
+// Two x-adjacent cells per thread: a tile is 64 x 8 or 64 x 16 cells (32 x 8
+// threads of one or two rows each, k1_rows).  Halo rows are loaded as aligned
 // pairs into shared rows padded so the pairs stay aligned (index 0 pad, 1 west
 // halo, 2..65 tile, 66 east halo); the two edge columns are scalar loads.
 // Only the thread's own cells need the mask (Ap = 0 in a solid cell), so it
 // is read straight from global memory.  Pairs need an even nx; odd nx uses
 // scalar loads.
 constexpr int PX = 64;          // tile width
-// rows a thread: one, so that four CTAs of 64 registers fit an SM (two rows and
-// three CTAs of 80 registers: 254 ms a plain FP64 solve at 256^3, against 244; five
-// CTAs spill: 285)
-constexpr int RPT = 1;
-constexpr int PY = 8 * RPT;     // tile height
 constexpr int PW = PX + 4;      // padded shared row
-constexpr int PHY = PY + 2;     // rows with halo
-constexpr int PROWS = (PHY + 7) / 8;  // halo rows per thread (2)
+// Rows a thread.  FP64 with exact neighbour sums is bound by latency: one row, so
+// that four CTAs of 64 registers fit an SM (two rows and three CTAs of 80 registers:
+// 254 ms a plain FP64 solve at 256^3, against 244; five CTAs spill: 285).  FP64 with
+// adds is bound by the FP64 pipe and FP32 by its loads: two, for fewer halo rows
+// (FP32 281x256x250 254 us an iteration with one row, 212 with two; FP64 160x144x155
+// anisotropic with walls 203 and 197).
+__host__ __device__ constexpr int k1_rows(bool f64, bool iso) { return f64 && iso ? 1 : 2; }
 
 template <typename T> struct V2of;
 template <> struct V2of<double> { typedef double2 type; };
@@ -271,11 +272,15 @@ __device__ __forceinline__ void store_own(T *__restrict__ pnew, T *__restrict__ 
 }
 
 template <typename T, bool MASK, bool ISO>
-__global__ void __launch_bounds__(FNT, 4) k1_search2(const GeoL G, const T *__restrict__ r, const T *__restrict__ pold,
+__global__ void __launch_bounds__(FNT, sizeof(T) == 8 && !ISO ? 3 : 4) k1_search2(const GeoL G, const T *__restrict__ r, const T *__restrict__ pold,
                                                   T *__restrict__ pnew, T *__restrict__ Ap, T *__restrict__ x,
                                                   const uint8_t *__restrict__ mask, DevState *st, double *partials,
                                                   int kz) {
   typedef typename V2of<T>::type V2;
+  constexpr int RPT = k1_rows(sizeof(T) == 8, ISO);
+  constexpr int PY = 8 * RPT;           // tile height
+  constexpr int PHY = PY + 2;           // rows with halo
+  constexpr int PROWS = (PHY + 7) / 8;  // halo rows per thread
   __shared__ T s_dL[27], s_inv[27];
   __shared__ __align__(16) T sp[4][PHY][PW];
   __shared__ double s_red[FNT / 32];

@@ -67,7 +67,7 @@ struct bbpp_ctx {
   int fkz = 1;         // z planes per CTA of the residual kernel
   dim3 fgrid;          // grid of the residual kernel (32x16 tiles)
   int pkz[2] = {1, 1};  // z planes per CTA of the search kernel [FP32, FP64]
-  dim3 pgrid[2];        // grid of the search kernel (64x8 tiles) [FP32, FP64]
+  dim3 pgrid[2];        // grid of the search kernel (64 x 8 k1_rows tiles) [FP32, FP64]
   int egrid = 1;       // elementwise grid (1-D)
   size_t nparts = 0;   // capacity of partials (per sum)
   cudaStream_t own_stream = nullptr, stream = nullptr;

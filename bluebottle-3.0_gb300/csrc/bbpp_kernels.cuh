@@ -51,7 +51,7 @@ __device__ __noinline__ static double wall_rz(double rz, double w, double rd) { 
 // walls, as one exact sum on the integer pipe (xsum6).
 // Bound by the FP64 pipe with FP64 adds (13 instructions a cell; 426 us at 256^3);
 // with the integer sums, (r,z) as (r,r) plus the wall cells' part, and a plane's
-// loads in flight while the one before is computed it takes 276 us.
+// loads in flight while the one before is computed it takes 300 us.
 template <typename TXT, typename TR, bool MASK>
 __global__ void __launch_bounds__(NT) k_resid(const Geo G, const TXT *__restrict__ xin,
                                               const TXT *__restrict__ rhs, TR *__restrict__ rout,

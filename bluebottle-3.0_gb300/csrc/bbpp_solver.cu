@@ -142,7 +142,7 @@ __global__ void k_invm(const Geo G, double *invM) {
 // FP32 places clearly inside or outside (all but those within its error of the
 // surface) skip it.  Bound by the FP64 pipe before: a CTA per image, whose 256
 // threads each found its box and tested every cell in FP64, took 630 us for 1000
-// spheres of radius 6 at 256^3; this takes 17.
+// spheres of radius 6 at 256^3; this takes 25.
 struct SphereBox {
   int i0, j0, k0, bx, by, n;  // n = 0: no cell of the grid
   double X, Y, Z;             // centre less the origin
@@ -253,12 +253,15 @@ static void stencil_shape(bbpp_ctx *ctx) {
   }
   for (int prec = 0; prec < 2; prec++) {
     // one full wave of resident CTAs of the search kernel of this precision
-    const int fx = (G.nx + PX - 1) / PX, fy = (G.ny + PY - 1) / PY;
+    const int py = 8 * k1_rows(prec == 1, ctx->GL.iso != 0);
+    const int fx = (G.nx + PX - 1) / PX, fy = (G.ny + py - 1) / py;
     int pf = 0;
-    if (prec)
+    if (!prec)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k1_search2<float, true, true>, FNT, 0);
+    else if (ctx->GL.iso)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k1_search2<double, true, true>, FNT, 0);
     else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k1_search2<float, true, true>, FNT, 0);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k1_search2<double, true, false>, FNT, 0);
     if (pf < 1) pf = 1;
     int kzf = 0;
     const int nzf = bbpp_z_chunks((long long)fx * fy, G.nz, (long long)ctx->sms * pf, 8, &kzf);
@@ -1268,7 +1271,7 @@ __device__ __forceinline__ double mul_pow2(double v, double m, int k) {
 // PP_rhs (src/solver_kernel.cu:152-173) on dense face arrays: rhs = -(rho/dt)
 // div u*, the reference's evaluation order without contraction.  Bound by the FP64
 // pipe (9 instructions a cell); on spacings of 1 / 2^k, the usual ones, six
-// (POW2): at 256^3 333 us before, 205 now.
+// (POW2): at 256^3 333 us before, 244 now.
 template <bool POW2>
 __global__ void __launch_bounds__(256) k_rhs_div(const Geo G, double idx, double idy, double idz, int kx, int ky,
                                                  int kz, double rho_idt, const double *__restrict__ u,

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstring>
+
 namespace bbpp {
 
 // Programmatic dependent launch: wait until the preceding kernel of the stream
@@ -72,9 +74,35 @@ struct DevState {
   // number of steps; residual kernels write z = r / dL in place of r
   double pair[4];
   int pair_steps;
-  int pair_fresh;  // the pair (counted by fq) whose search direction is z, not p
+  int pair_fresh;  // the pair (counted by fq) that starts along z, not p
+  int pair_anew;   // the pair (counted by fq), if any, whose dots decided to go along z
   int zform;
+  double rz_next;  // (r,z) that the expansions of a pair expect at the next one's start
 };
+
+// Comparisons of (r,z) values by their high words: an FP64 instruction, taken or not,
+// costs the one thread that decides at the end of a kernel 16 cycles and more.
+// What one step of an expansion must leave of (r,z) for beta to be used: 2^-kBetaKeeps.
+constexpr int kBetaKeeps = 10;
+__host__ __device__ inline int hi_word(double v) {
+#ifdef __CUDA_ARCH__
+  return __double2hiint(v);
+#else
+  long long b;
+  memcpy(&b, &v, 8);
+  return (int)(b >> 32);
+#endif
+}
+// a >= 2^-k b > 0 to 20 bits; false for NaN and infinities
+__host__ __device__ inline bool keeps(double a, double b, int k) {
+  const int ha = hi_word(a), hb = hi_word(b);
+  return hb > k << 20 && ha >= hb - (k << 20) && ha < 0x7ff00000;
+}
+// a and b positive and within a tenth of each other (20 bits; 0.05 next to a power of two)
+__host__ __device__ inline bool alike(double a, double b) {
+  const int ha = hi_word(a), hb = hi_word(b), d = ha - hb;
+  return ha > 0 && hb > 0 && ha < 0x7ff00000 && d <= 104858 && d >= -104858;
+}
 
 __device__ __forceinline__ void trace_put(double *buf, int n, int i, double v) {
   if (buf && i >= 0 && i < n) buf[i] = v;

@@ -891,8 +891,10 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
 // random solid cells at 160^3 to 1e-8: 5649 iterations without, under 100 with it.
 constexpr double kLostBeta = 4.0;
 // pairs: p is already formed when the residual comes; rz as the recursion had it
+// (a restart that the pair itself asked for stands)
 __device__ __forceinline__ void pair_restart(DevState *st, double rz1, double rz) {
-  st->pair_fresh = (rz1 <= 1.5 * rz && rz <= 1.5 * rz1) ? -1 : st->fq;
+  if (!(rz1 <= 1.5 * rz && rz <= 1.5 * rz1)) st->pair_fresh = st->fq;
+  st->rz_next = rz1;
 }
 
 // The device state after a residual: init (mode 0), replacement at a
@@ -921,7 +923,7 @@ __device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3
     } else if (mode == 1) {
       st->replacements += 1;
       st->dlag = 0;  // x was settled before this residual
-      if (st->zform) pair_restart(st, rz1, st->rz * st->pair[1] * (st->pair_steps == 2 ? st->pair[3] : 1.0));
+      if (st->zform) pair_restart(st, rz1, st->rz_next);
       finish_iteration(st, rz1, rr1, !st->zform);  // a pair's kernels have counted theirs
       if (st->beta > kLostBeta) st->beta = 0.0;
       st->rr_ref = rr1;

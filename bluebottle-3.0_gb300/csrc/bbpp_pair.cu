@@ -6,7 +6,7 @@
 // The vectors are z = r / dL (dL the diagonal of L; r = z away from walls), p
 // and x.  With w = L p, q = w / dL, t = L q, s = L z, two iterations need only
 // the products (r,z), (r,r), (p,w), (z,w), (q,w), (z,s), (z,t), (q,t), (s,s/dL),
-// (s,t/dL), (t,t/dL): they give alpha and beta of both iterations (pair_coefs).
+// (s,t/dL), (t,t/dL): they give alpha and beta of both iterations (pair_plan).
 //   k_pair<false>  forms w, t and s on the fly and sums the products: reads z, p
 //                  and the mask (9 B/cell), writes nothing;
 //   k_pair<true>   forms them again and applies both steps: reads z, p, x and
@@ -131,31 +131,83 @@ __device__ __forceinline__ void add_to(Pairf &a, float v) {
 }  // namespace
 
 namespace bbpp {
-// alpha and beta of the pair's two iterations from the products of its start;
-// d: (r,z), (r,r) - (r,z), (p,w), (z,w), (q,w), (z,s), (z,t), (q,t), (s,s'), (s,t'),
-// (t,t') with ' = / dL.  Symmetry of L gives the others: (q,s) = (z,t),
-// (p,s) = (z,w), (p,t) = (q,w).
-__host__ __device__ inline void pair_coefs(const double *d, double &a0, double &b0, double &a1, double &b1) {
+// A pair's steps from the products of its start; d: (r,z), (r,r) - (r,z), (p,w),
+// (z,w), (q,w), (z,s), (z,t), (q,t), (s,s'), (s,t'), (t,t') with ' = / dL.  Symmetry
+// of L gives the others: (q,s) = (z,t), (p,s) = (z,w), (p,t) = (q,w).
+struct PairPlan {
+  double a0, b0, a1, b1;
+  int steps;   // 1 or 2
+  bool anew;   // this pair's search direction is z, not p
+  bool fresh;  // the next pair's is
+  double rz;   // (r,z) after the steps, by the expansions
+};
+// The products are FP32 sums (relative errors of some 1e-6), so an expansion is
+// known to that part of its largest term: what a step leaves, (r,z) after it, has
+// no digits where a step takes nearly all of the residual (a right-hand side of few
+// eigenvectors, a mask of isolated cells), and 0 / 0 follows where it takes all.
+//   A second step is taken only where each of the two leaves 2^-kStepKeeps of (r,z);
+//   else one step, and the next pair's exact sums decide.
+//   One step must leave 2^-kBetaKeeps for beta to be used; else p = z next.
+//   The exact (r,z) of a pair's start lies within a tenth of what the pair before
+//   expected; else p is conjugate to nothing, and this pair takes one step along z
+//   (whose products are among the eleven: w = s, q = s / dL).
+// Solves of spectral and uniform right-hand sides with 0 to 80% solid cells expect
+// (r,z) to 1e-5 or better and take two steps throughout (numpy model at 64^3).
+// The tests read high words, and the rare restart is a call: one thread works here
+// at the end of every dots kernel, and an FP64 instruction, taken or not, costs it 16
+// cycles and more (with FP64 compares and the restart in line 2 us a pair).
+constexpr int kStepKeeps = 5;
+
+// one step along z
+__host__ __device__ __noinline__ static void pair_restart_plan(const double *d, PairPlan &o) {
+  const double rz = d[0], zs = d[5], ss = d[8];
+  o.a0 = rz / zs;
+  o.rz = rz - 2.0 * o.a0 * zs + o.a0 * o.a0 * ss;
+  o.fresh = !keeps(o.rz, rz, kBetaKeeps);
+  o.b0 = o.fresh ? 0.0 : o.rz / rz;
+  o.steps = 1;
+  o.anew = true;
+}
+__host__ __device__ inline PairPlan pair_plan(const double *d, bool fresh, double expected) {
   const double rz = d[0], pw = d[2], zw = d[3], qw = d[4], zs = d[5], zt = d[6], qt = d[7], ss = d[8], st = d[9],
                tt = d[10];
-  a0 = rz / pw;
-  const double rz1 = rz - 2.0 * a0 * zw + a0 * a0 * qw;
-  b0 = rz1 / rz;
+  PairPlan o;
+  o.a0 = rz / pw;
+  const double a0 = o.a0, rz1 = rz - 2.0 * a0 * zw + a0 * a0 * qw, b0 = rz1 / rz;
   // p1 = z - a0 q + b0 p, w1 = L p1 = s - a0 t + b0 w
   const double zw1 = zs - 2.0 * a0 * zt + a0 * a0 * qt + b0 * (zw - a0 * qw);  // (z1, w1)
   const double pw1 = zw1 + b0 * (zw - a0 * qw + b0 * pw);                      // (p1, w1)
   const double ww1 = ss + a0 * a0 * tt + b0 * b0 * qw - 2.0 * a0 * st + 2.0 * b0 * (zt - a0 * qt);  // (w1, w1 / dL)
-  a1 = rz1 / pw1;
-  const double rz2 = rz1 - 2.0 * a1 * zw1 + a1 * a1 * ww1;
-  b1 = rz2 / rz1;
+  o.a1 = rz1 / pw1;
+  const double rz2 = rz1 - 2.0 * o.a1 * zw1 + o.a1 * o.a1 * ww1;
+  o.b1 = rz2 / rz1;
+  const bool two = keeps(rz1, rz, kStepKeeps) && hi_word(pw1) > 0 && keeps(rz2, rz1, kStepKeeps);
+  o.steps = two ? 2 : 1;
+  o.rz = two ? rz2 : rz1;
+  o.fresh = !keeps(rz1, rz, kBetaKeeps);
+  o.b0 = o.fresh ? 0.0 : b0;
+  o.anew = fresh;
+  if (!fresh && !(alike(rz, expected) && hi_word(pw) > 0)) pair_restart_plan(d, o);
+  return o;
 }
 }  // namespace bbpp
 
+// What the end of a dots kernel reads of the state, at once: one load after another,
+// between the stores, would take an L2 latency each.
+struct PairIn {
+  int iter, stop, max_iter, fq, fresh, maxgap, last_rep;
+  double tol2bb, expected, rep_d2, rr_ref;
+};
+__device__ __forceinline__ PairIn pair_in(const DevState *st) {
+  return {st->iter,     st->stop,    st->max_iter, st->fq,     st->pair_fresh, st->rep_maxgap,
+          st->last_rep, st->tol2bb,  st->rz_next,  st->rep_d2, st->rr_ref};
+}
+
 // The end of a dots kernel: convergence of the residual at the pair's start,
-// then the coefficients and the number of steps (1 where a second would pass a
+// then the coefficients and the number of steps (1 also where a second would pass a
 // checkpoint or the iteration limit).
-__device__ static void pair_finish(DevState *st, const double *d, int replace_every) {
-  const int it = st->iter;
+__device__ static void pair_finish(DevState *st, const PairIn &in, const double *d, int replace_every) {
+  const int it = in.iter;
   const double rz = d[0], rr = d[0] + d[1];
   st->rz_last = rz;
   st->rr = rr;
@@ -164,28 +216,30 @@ __device__ static void pair_finish(DevState *st, const double *d, int replace_ev
     st->done = DONE_NAN;
     return;
   }
-  if (it > 0 && (st->stop == 0 ? rz : rr) <= st->tol2bb) {
-    st->done = it > st->max_iter ? DONE_MAX_ITER : (st->stop == 0 ? DONE_CONVERGED : DONE_PENDING);
+  if (it > 0 && (in.stop == 0 ? rz : rr) <= in.tol2bb) {
+    st->done = it > in.max_iter ? DONE_MAX_ITER : (in.stop == 0 ? DONE_CONVERGED : DONE_PENDING);
     return;
   }
-  if (it > st->max_iter) {
+  if (it > in.max_iter) {
     st->done = DONE_MAX_ITER;
     return;
   }
-  double a0, b0, a1, b1;
-  pair_coefs(d, a0, b0, a1, b1);
-  const int n = ((it + 1) % replace_every == 0 || it + 1 > st->max_iter) ? 1 : 2;
+  const PairPlan o = pair_plan(d, in.fresh == in.fq, in.expected);
+  const int n = ((it + 1) % replace_every == 0 || it + 1 > in.max_iter) ? 1 : o.steps;
   st->pAp = d[2];
-  st->pair[0] = a0;
-  st->pair[1] = b0;
-  st->pair[2] = a1;
-  st->pair[3] = b1;
+  st->pair[0] = o.a0;
+  st->pair[1] = o.b0;
+  st->pair[2] = o.a1;
+  st->pair[3] = o.b1;
   st->pair_steps = n;
+  st->pair_anew = o.anew ? in.fq : -1;
+  st->rz_next = n == o.steps ? o.rz : rz * o.b0;
   st->iter = it + n;
-  st->fq += 1;
+  st->fq = in.fq + 1;
+  if (o.fresh) st->pair_fresh = in.fq + 1;
   // a checkpoint after this pair: replace the residual?
   st->rep_now = (it + n) % replace_every == 0 &&
-                ((st->rep_d2 <= 0.0) || (rr <= st->rep_d2 * st->rr_ref) || (it + n - st->last_rep >= st->rep_maxgap));
+                ((in.rep_d2 <= 0.0) || (rr <= in.rep_d2 * in.rr_ref) || (it + n - in.last_rep >= in.maxgap));
 }
 
 // STEP: apply the steps; else sum the products.  WXY: walls in x or y (cells of
@@ -203,8 +257,8 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   __shared__ int s_last;
   __shared__ int s_piece[2][8][3], s_np[4];
   if (*(volatile int *)&st->done) return;
-  // the first pair, and a restart after a replaced residual: p = z
-  const bool fresh = *(volatile int *)&st->pair_fresh == *(volatile int *)&st->fq - (STEP ? 1 : 0);
+  // the first pair, and restarts (pair_plan, pair_restart): p = z
+  const bool fresh = *(volatile int *)(STEP ? &st->pair_anew : &st->pair_fresh) == *(volatile int *)&st->fq - (STEP ? 1 : 0);
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
   const bool skip_one = *(volatile int *)&st->inject && blockIdx.x == 0 && blockIdx.y == 0;
@@ -677,6 +731,7 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  const PairIn in = pair_in(st);
   double *sd = reinterpret_cast<double *>(smem_raw);
   for (int k = tid >> 5; k < NDOT; k += nth >> 5) {
     double a = 0.0;
@@ -687,7 +742,7 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   __syncthreads();
   if (tid == 0) {
     st->ticket = 0;
-    pair_finish(st, sd, replace_every);
+    pair_finish(st, in, sd, replace_every);
   }
 }
 

@@ -77,7 +77,7 @@ struct DevState {
   int pair_fresh;  // the pair (counted by fq) that starts along z, not p
   int pair_anew;   // the pair (counted by fq), if any, whose dots decided to go along z
   int zform;
-  double rz_next;  // (r,z) that the expansions of a pair expect at the next one's start
+  double rz_next;  // (r,z) that the expansions of a pair or a fused kernel expect next
 };
 
 // Comparisons of (r,z) values by their high words: an FP64 instruction, taken or not,

@@ -413,6 +413,17 @@ struct FusedMaps {
   CUtensorMap r_rows, r_row, a_rows, a_row, p_rows, p_row;
 };
 
+// The next beta from the expansion, c1 = (Ap, z), c2 = (Ap, Ap / dL).  Its terms are
+// FP32 sums, so beta has no digits where a step takes nearly all of the residual (a
+// right-hand side of few eigenvectors), and a p of such a beta is conjugate to
+// nothing, which shows where the exact (r,z) is not what was expected of it: p = z then.
+__device__ __forceinline__ void expand_beta(DevState *st, double rz, double alpha, double c1, double c2, bool lag) {
+  const double next = rz - 2.0 * alpha * c1 + alpha * alpha * c2, expected = st->rz_next;
+  const bool use = keeps(next, rz, kBetaKeeps) && (!lag || expected == 0.0 || alike(rz, expected));
+  st->beta = use ? next / rz : 0.0;
+  st->rz_next = use ? next : 0.0;
+}
+
 template <int NPT, bool MASK, bool ISO>
 __global__ void __launch_bounds__(TNT) k1_fused(const GeoL G, const __grid_constant__ FusedMaps M,
                                                 float *__restrict__ rout, float *__restrict__ pnew,
@@ -709,10 +720,10 @@ __global__ void __launch_bounds__(TNT) k1_fused(const GeoL G, const __grid_const
     // recursive residual has met TRUE_REL: the confirmation folds it in)
     if (st->done == RUNNING || st->done == DONE_PENDING) {
       const double rz = st->rz, pap = tot[0];
-      const double a = rz / pap;
+      const double a = rz == 0.0 ? 0.0 : rz / pap;  // p = z = 0 after a step that took all
       st->pAp = pap;
       st->alpha = a;
-      st->beta = (rz - 2.0 * a * tot[3] + a * a * tot[4]) / rz;
+      expand_beta(st, rz, a, tot[3], tot[4], lag);
       st->first = 0;
       st->dlag = 1;
       decide_replacement(st);
@@ -1083,10 +1094,10 @@ __global__ void __launch_bounds__(WS_THREADS, 3) k1_fused_ws(const GeoL G, const
     st->dlag = 0;
     if (st->done == RUNNING || st->done == DONE_PENDING) {
       const double rz = st->rz, pap = tot[0];
-      const double a = rz / pap;
+      const double a = rz == 0.0 ? 0.0 : rz / pap;  // p = z = 0 after a step that took all
       st->pAp = pap;
       st->alpha = a;
-      st->beta = (rz - 2.0 * a * tot[3] + a * a * tot[4]) / rz;
+      expand_beta(st, rz, a, tot[3], tot[4], lag);
       st->first = 0;
       st->dlag = 1;
       decide_replacement(st);

@@ -35,7 +35,9 @@ def modes(n, names):
 
 
 def solve(monkeypatch, form, g, b, mask, tol):
-    """form: pair, fused, two (search + update kernels) or resident."""
+    """form: pair, fused, fused_ws, two (search + update kernels) or resident."""
+    if form == "fused_ws":
+        monkeypatch.setenv("BBPP_FUSED_WS", "1")
     monkeypatch.setenv("BBPP_PERSIST", "1" if form == "resident" else "0")
     monkeypatch.setenv("BBPP_PAIR", "1" if form == "pair" else "0")
     s = bbpp.Solver(g)
@@ -46,7 +48,7 @@ def solve(monkeypatch, form, g, b, mask, tol):
     return x, rep
 
 
-FORMS = [("pair", 48), ("pair", 64)]
+FORMS = [("pair", 48), ("pair", 64), ("fused", 64), ("fused_ws", 64)]
 
 
 @pytest.mark.parametrize("tol", [1e-4, 1e-6, 1e-8, 1e-10])

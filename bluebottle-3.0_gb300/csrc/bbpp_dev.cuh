@@ -77,7 +77,7 @@ struct DevState {
   int pair_fresh;  // the pair (counted by fq) that starts along z, not p
   int pair_anew;   // the pair (counted by fq), if any, whose dots decided to go along z
   int zform;
-  double rz_next;  // (r,z) that the expansions of a pair or a fused kernel expect next
+  double rz_next;  // the recursion's (r,z): the last one's, or what a pair or a fused kernel expects next
 };
 
 // Comparisons of (r,z) values by their high words: an FP64 instruction, taken or not,
@@ -270,6 +270,7 @@ __device__ __forceinline__ void finish_iteration(DevState *st, double rz1, doubl
   int it = st->iter + (count_iter ? 1 : 0);
   st->iter = it;
   st->rz_last = rz1;
+  st->rz_next = rz1;
   st->rr = rr1;
   bool conv = (st->stop == 0) ? (rz1 <= st->tol2bb) : (rr1 <= st->tol2bb);
   if (conv) {

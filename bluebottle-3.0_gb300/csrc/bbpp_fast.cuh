@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(FNT) k_settle(const GeoL G, T *__restrict__ x,
 }
 
 // --------------------------------------------------------------- residual --
-__device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3], int mode);
+__device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3], int mode, bool fp32);
 
 // r = bscale rhs - L x on fluid cells, r = 0 (and x = 0 with zero_solid_x) on
 // solid cells.  TXT: type of x and rhs, TR: type of r.  Dots in FP64 of the
@@ -881,26 +881,33 @@ __global__ void __launch_bounds__(FNT, 3) k_resid_s(const GeoL G, TXT *__restric
   double v[3] = {rr + corr, rr, bb}, tot[3];
   const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
   const unsigned int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  if (last_cta_reduce<3>(v, partials, st, nb, bid, s_red, tot) && tid == 0) resid_finish(st, tot, mode);
+  if (last_cta_reduce<3>(v, partials, st, nb, bid, s_red, tot) && tid == 0)
+    resid_finish(st, tot, mode, sizeof(TXT) != sizeof(TR));
 }
 
-// A replaced residual that is not the one the recursion carried (FP32 lost it: a
-// solve that converges by more than 1e7 between two replacements) leaves a search
-// direction that is not conjugate to it, and CG never recovers from that: the
-// iterations stall or diverge.  They restart from the residual instead.  10% of
-// random solid cells at 160^3 to 1e-8: 5649 iterations without, under 100 with it.
-constexpr double kLostBeta = 4.0;
-// pairs: p is already formed when the residual comes; rz as the recursion had it
-// (a restart that the pair itself asked for stands)
-__device__ __forceinline__ void pair_restart(DevState *st, double rz1, double rz) {
-  if (!(rz1 <= 1.5 * rz && rz <= 1.5 * rz1)) st->pair_fresh = st->fq;
-  st->rz_next = rz1;
+// An FP32 iteration whose recursion has lost its residual: the replaced one is far from
+// the one it carried, the search direction is not conjugate to it, and CG does not
+// recover from that (it stalls, or ends at p = 0: the FP32 operator's steps overshoot
+// FP64's by 1e-8, so a p that is kept can cancel z).  It restarts from the residual.
+// Where the recursion's (r,z) of the same iteration is known (a confirmation, a pair's
+// checkpoint), a factor 1.5 apart is lost.  The one-step forms skip the recursion's
+// update at a checkpoint that replaces: there a replaced (r,z) of more than kLostBeta
+// times the last iteration's is lost if the recursion had reduced (r,r) by kLostGain
+// since the last replacement: a CG step's own beta is above 4 in the first iterations
+// only (5 to 27 with smooth right-hand sides and spheres, none above 1.3 from the
+// tenth on), when the recursion has gained nothing that FP32 could lose.
+// 10% of random solid cells at 160^3 to 1e-8: 5649 iterations without, under 100 with
+// it; one eigenvector at 48^3 to 1e-6: above 400 and 7.
+// FP64 iterations (the reference's method) keep every direction.
+constexpr double kLostBeta = 4.0, kLostGain = 1e-4;
+__device__ __forceinline__ bool lost(double rz1, double expected) {
+  return !(rz1 <= 1.5 * expected && expected <= 1.5 * rz1);
 }
 
 // The device state after a residual: init (mode 0), replacement at a
 // checkpoint (1) or confirmation of a recursive convergence (2).  tot: (r,z),
-// (r,r), (rhs,rhs).
-__device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3], int mode) {
+// (r,r), (rhs,rhs).  fp32: the residual of an FP32 iteration, from an FP64 x.
+__device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3], int mode, bool fp32) {
   {
     const double rz1 = tot[0], rr1 = tot[1];
     if (mode == 0) {  // init: thresholds from (rhs,rhs) of the unscaled rhs
@@ -923,9 +930,10 @@ __device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3
     } else if (mode == 1) {
       st->replacements += 1;
       st->dlag = 0;  // x was settled before this residual
-      if (st->zform) pair_restart(st, rz1, st->rz_next);
+      const double rr0 = st->rr;  // an iteration earlier
+      if (st->zform && lost(rz1, st->rz_next)) st->pair_fresh = st->fq;
       finish_iteration(st, rz1, rr1, !st->zform);  // a pair's kernels have counted theirs
-      if (st->beta > kLostBeta) st->beta = 0.0;
+      if (fp32 && st->beta > kLostBeta && rr0 <= kLostGain * st->rr_ref) st->beta = 0.0;
       st->rr_ref = rr1;
       st->last_rep = st->iter;
     } else {  // confirm
@@ -940,10 +948,11 @@ __device__ __forceinline__ void resid_finish(DevState *st, const double (&tot)[3
       } else if (isnan(rz1)) {
         st->done = DONE_NAN;
       } else {
-        if (st->zform) pair_restart(st, rz1, st->rz);
-        st->beta = rz1 / st->rz;
-        if (st->beta > kLostBeta) st->beta = 0.0;
+        const bool anew = fp32 && lost(rz1, st->rz_next);
+        if (anew && st->zform) st->pair_fresh = st->fq;
+        st->beta = anew ? 0.0 : rz1 / st->rz;
         st->rz = rz1;
+        st->rz_next = rz1;
         st->done = (st->iter > st->max_iter) ? DONE_MAX_ITER : RUNNING;
       }
     }
@@ -1087,7 +1096,7 @@ __global__ void __launch_bounds__(FNT) k_resid_ff(const GeoL G, double *__restri
   double v[3] = {(double)rr + (double)corr, (double)rr, (double)bb}, tot[3];
   const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
   const unsigned int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  if (last_cta_reduce<3>(v, partials, st, nb, bid, s_red, tot) && tid == 0) resid_finish(st, tot, mode);
+  if (last_cta_reduce<3>(v, partials, st, nb, bid, s_red, tot) && tid == 0) resid_finish(st, tot, mode, true);
 }
 
 }  // namespace bbpp

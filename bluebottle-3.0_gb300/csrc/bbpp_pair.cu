@@ -212,6 +212,7 @@ __device__ static void pair_finish(DevState *st, const PairIn &in, const double 
   st->rz_last = rz;
   st->rr = rr;
   st->rz = rz;
+  st->rz_next = rz;
   if (isnan(rz)) {
     st->done = DONE_NAN;
     return;
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   __shared__ int s_last;
   __shared__ int s_piece[2][8][3], s_np[4];
   if (*(volatile int *)&st->done) return;
-  // the first pair, and restarts (pair_plan, pair_restart): p = z
+  // the first pair, and restarts (pair_plan, resid_finish): p = z
   const bool fresh = *(volatile int *)(STEP ? &st->pair_anew : &st->pair_fresh) == *(volatile int *)&st->fq - (STEP ? 1 : 0);
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;

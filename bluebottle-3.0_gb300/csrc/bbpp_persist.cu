@@ -1005,6 +1005,7 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
       if (!s_bad) {
         st->rz = rz;
         st->rz_last = rz_last;
+        st->rz_next = rz_last;
         st->rr = rr_last;
         st->pAp = pap;
         st->alpha = s_alpha;

@@ -48,7 +48,8 @@ def solve(monkeypatch, form, g, b, mask, tol):
     return x, rep
 
 
-FORMS = [("pair", 48), ("pair", 64), ("fused", 64), ("fused_ws", 64)]
+FORMS = [("pair", 48), ("pair", 64), ("fused", 64), ("fused_ws", 64), ("two", 48), ("two", 64),
+         ("resident", 48), ("resident", 64)]
 
 
 @pytest.mark.parametrize("tol", [1e-4, 1e-6, 1e-8, 1e-10])

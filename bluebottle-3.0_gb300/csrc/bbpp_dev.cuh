@@ -34,6 +34,12 @@ enum DoneCode : int {
   DONE_TIMEOUT = 6   // a bounded wait inside a kernel ran out
 };
 
+// Test hooks of bbpp_debug_wait: waits that run out, launches that are refused.
+enum Inject : int {
+  INJECT_COPIES = 1,     // FP32: the first CTA leaves one plane's copies out (the resident one's last CTA an exchange)
+  INJECT_LAST_WAIT = 2,  // resident: the last CTA takes its last wait for run out
+};
+
 // Device-resident scalar state of one PCG solve.
 struct DevState {
   double bb;       // (rhs, rhs)
@@ -62,7 +68,7 @@ struct DevState {
   int rep_maxgap;
   int last_rep;
   int rep_now;
-  int inject;            // test hook: 1 = the first TMA search CTA skips the copies of one plane
+  int inject;            // test hook of bbpp_debug_wait (Inject)
   long long wait_ns;     // bound of a device-side wait (0: one second)
   int fq;                // fused iteration kernels completed in this solve
   // alpha_k and beta_k of iterations 1 .. trace_n (index k - 1), recorded by

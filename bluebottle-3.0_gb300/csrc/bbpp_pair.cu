@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   const bool fresh = *(volatile int *)(STEP ? &st->pair_anew : &st->pair_fresh) == *(volatile int *)&st->fq - (STEP ? 1 : 0);
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
-  const bool skip_one = *(volatile int *)&st->inject && blockIdx.x == 0 && blockIdx.y == 0;
+  const bool skip_one = *(volatile int *)&st->inject == INJECT_COPIES && blockIdx.x == 0 && blockIdx.y == 0;
   load_tabs<float>(G, s_dL, s_inv);
 
   const int tid = threadIdx.x, lane = tid & 31;

@@ -328,7 +328,8 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
   // test hook (FP32 solves): the last CTA leaves its first exchange out
-  const bool silent0 = sizeof(T) == 4 && *(volatile int *)&st->inject && blockIdx.x == (unsigned)B.nb - 1u;
+  const int inject = blockIdx.x == (unsigned)B.nb - 1u ? *(volatile int *)&st->inject : 0;
+  const bool silent0 = sizeof(T) == 4 && inject == INJECT_COPIES;
   const int tid = threadIdx.x;
   if (tid < 27) s_inv[tid] = sizeof(T) == 8 ? (T)G.invL[tid] : (T)G.finvL[tid];
   if (tid < 27) s_dm1[tid] = (sizeof(T) == 8 ? (T)G.dL[tid] : (T)G.fdL[tid]) - T(1);
@@ -981,6 +982,10 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
     }
   }
 
+  if (inject == INJECT_LAST_WAIT && s_done != RUNNING) {
+    if (tid == 0) s_bad = 1;
+    __syncthreads();
+  }
   if (!s_bad) {
     T *po = (it & 1) ? p1 : p0;
     for (int col = col0; col < ncol; col += NTH) {
@@ -1016,7 +1021,8 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
         st->dlag = checkpoint ? 1 : 0;
         st->iter = checkpoint ? it - 1 : it;
         if (checkpoint) decide_replacement(st);
-        else st->done = s_done;
+        // another CTA's wait may have run out in the last exchange: that stands
+        else if (s_done != RUNNING) atomicCAS(&st->done, (int)RUNNING, s_done);
       }
     }
   }

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(TNT) k1_tma(const GeoL G, const __grid_constan
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
   // test hook: CTA (0,0) leaves one plane's copies unissued, so that its wait
   // for them runs out and the solve ends with DONE_TIMEOUT
-  const bool skip_one = *(volatile int *)&st->inject && blockIdx.x == 0 && blockIdx.y == 0;
+  const bool skip_one = *(volatile int *)&st->inject == INJECT_COPIES && blockIdx.x == 0 && blockIdx.y == 0;
   load_tabs<float>(G, s_dL, s_inv);
   // L2 policies: the mask, read by every search kernel, stays (evict_last);
   // p, Ap and x stream through (evict_first); r keeps the normal priority
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(TNT) k1_fused(const GeoL G, const __grid_const
   const float alpha = lag ? (float)(*(volatile double *)&st->alpha) : 0.f;
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
-  const bool skip_one = *(volatile int *)&st->inject && blockIdx.x == 0 && blockIdx.y == 0;
+  const bool skip_one = *(volatile int *)&st->inject == INJECT_COPIES && blockIdx.x == 0 && blockIdx.y == 0;
   load_tabs<float>(G, s_dL, s_inv);
   const unsigned long long pol_n = l2_policy(0), pol_stream = l2_policy(l2hint ? 1 : 0);
   const unsigned long long pol_mask = l2_policy(l2hint ? 2 : 0);
@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(WS_THREADS, 3) k1_fused_ws(const GeoL G, const
   const float alpha = lag ? (float)(*(volatile double *)&st->alpha) : 0.f;
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
-  const bool skip_one = *(volatile int *)&st->inject && blockIdx.x == 0 && blockIdx.y == 0;
+  const bool skip_one = *(volatile int *)&st->inject == INJECT_COPIES && blockIdx.x == 0 && blockIdx.y == 0;
   load_tabs<float>(G, s_dL, s_inv);
   const unsigned long long pol_n = l2_policy(0), pol_stream = l2_policy(l2hint ? 1 : 0);
   const unsigned long long pol_mask = l2_policy(l2hint ? 2 : 0);

@@ -1,0 +1,43 @@
+"""Waits and launches of the resident iteration that fail (csrc/bbpp_persist.cu),
+by the host's and the kernels' test hooks: the solve says so, or goes on kernel
+by kernel, and the context stays usable.  Nothing faults, traps or hangs."""
+import numpy as np
+import pytest
+
+import bbpp
+from bbpp import problems
+
+pytestmark = pytest.mark.gpu
+LAST_WAIT = 2
+
+
+def problem(dims, bc, seed=3):
+    nx, ny, nz = dims
+    g = bbpp.Grid.make(nx, ny, nz, 1.0 / nx, 1.0 / ny, 1.0 / nz, problems.bc_tuple(bc))
+    rng = np.random.default_rng(seed)
+    mask = (rng.random(g.shape) < 0.05).astype(np.uint8)
+    b = rng.uniform(-1, 1, g.shape)
+    b[mask == 1] = 0
+    b[mask == 0] -= b[mask == 0].mean()
+    return g, mask, b
+
+
+ANY = (bbpp.CONVERGED, bbpp.WAIT_TIMEOUT)
+
+
+@pytest.mark.parametrize("precision", [bbpp.FP64, bbpp.FP32_IR])
+@pytest.mark.parametrize("dims", [(40, 33, 29), (128, 100, 90)])
+def test_a_wait_that_ran_out_is_not_overwritten(bbpp_lib, precision, dims):
+    """The last CTA's wait runs out in the exchange by which the others see the
+    solve converge: one box is not written back, so the solve must not pass for
+    converged.  Under the (r,z) rule no residual is formed again that would show it."""
+    g, mask, b = problem(dims, "ppn")
+    s = bbpp.Solver(g)
+    L = bbpp.lib()
+    for _ in range(4):
+        assert L.bbpp_debug_wait(s.handle, 0, LAST_WAIT) == 0
+        x, rep = s.solve_host(b, mask, tol=1e-8, precision=precision, stop=bbpp.STOP_REF_RZ, ok=ANY)
+        assert rep.status == bbpp.WAIT_TIMEOUT
+    assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
+    x, rep = s.solve_host(b, mask, tol=1e-8, precision=precision)
+    assert rep.status == bbpp.CONVERGED and rep.true_rel <= 1.01e-8

@@ -38,6 +38,7 @@ enum DoneCode : int {
 enum Inject : int {
   INJECT_COPIES = 1,     // FP32: the first CTA leaves one plane's copies out (the resident one's last CTA an exchange)
   INJECT_LAST_WAIT = 2,  // resident: the last CTA takes its last wait for run out
+  INJECT_REFUSED = 3,    // resident: the host takes the launch for refused
 };
 
 // Device-resident scalar state of one PCG solve.

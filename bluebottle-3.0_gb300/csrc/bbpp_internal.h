@@ -220,6 +220,7 @@ void bbpp_persist_init(bbpp_ctx *ctx);
 void bbpp_persist_free(bbpp_ctx *ctx);
 bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem);
 int bbpp_persist_begin(bbpp_ctx *ctx);
+bool bbpp_persist_refused(bbpp_ctx *ctx, int elem, cudaError_t e);
 template <typename T>
 int bbpp_persist(bbpp_ctx *ctx, const uint8_t *mask, T *r, T *const p[2], T *Ap, T *x, bbpp::DevState *st,
                  int replace_every);

@@ -1034,6 +1034,7 @@ struct bbpp_persist_state {
   bool ok[2] = {false, false};
   int nth[2] = {512, 512};
   bbpp_exchange *ex = nullptr;
+  bool refused = false;  // the last launch
 };
 
 namespace {
@@ -1195,6 +1196,18 @@ int bbpp_persist_begin(bbpp_ctx *ctx) {
   return 0;
 }
 
+// Was the resident launch refused (the last bbpp_persist, or, with e, the launch of a graph of it)?  Then the
+// context makes no more of them.
+bool bbpp_persist_refused(bbpp_ctx *ctx, int elem, cudaError_t e) {
+  bbpp_persist_state *t = ctx->persist;
+  if (!t->refused && e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return false;
+  cudaGetLastError();
+  ctx->err.clear();
+  t->refused = false;
+  t->ok[elem == 8 ? 1 : 0] = false;
+  return true;
+}
+
 template <typename T>
 int bbpp_persist(bbpp_ctx *ctx, const uint8_t *mask, T *r, T *const p[2], T *Ap, T *x, DevState *st,
                  int replace_every) {
@@ -1211,9 +1224,12 @@ int bbpp_persist(bbpp_ctx *ctx, const uint8_t *mask, T *r, T *const p[2], T *Ap,
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const cudaError_t e =
-      cudaLaunchKernelEx(&cfg, pick(T(0), ctx->persist->nth[k], B, mask != nullptr, ctx->GL.iso != 0), ctx->GL, B,
-                         p[0], p[1], r, Ap, x, mask, st, ctx->persist->ex, replace_every);
+      ctx->inject == INJECT_REFUSED
+          ? cudaErrorCooperativeLaunchTooLarge
+          : cudaLaunchKernelEx(&cfg, pick(T(0), ctx->persist->nth[k], B, mask != nullptr, ctx->GL.iso != 0), ctx->GL,
+                               B, p[0], p[1], r, Ap, x, mask, st, ctx->persist->ex, replace_every);
   if (e != cudaSuccess) {
+    ctx->persist->refused = e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported;
     bbpp_record_error(ctx, e, "k_persist", __LINE__);
     return BBPP_CUDA_ERROR;
   }

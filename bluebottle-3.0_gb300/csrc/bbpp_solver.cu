@@ -665,9 +665,10 @@ static int launch_resident(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *
                            DevState *st, int q, int replace_every) {
   const int qc = (q / replace_every + 1) * replace_every;
   const int rc = bbpp_persist<T>(ctx, mask, r, p, Ap, x, st, replace_every);
+  if (rc) return rc;  // nothing has run
   launch_update<T>(ctx, r, Ap, st, 1);
   launch_replace<T>(ctx, mask, x, rhs, r, p[qc & 1], st, RES_ITER);
-  return rc;
+  return 0;
 }
 
 // Capture (or reuse) the graph of iterations q0+1 .. q0+len for these buffers.
@@ -747,11 +748,13 @@ static int get_chunk_graph(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *
     const int gi = capture_chunk(
         ctx, key, len / replace_every,
         [&](int i) {
-          const int rl =
-              launch_resident<T>(ctx, mask, rhs, x, r, p, Ap, st, (i - 1) * replace_every, replace_every);
-          if (rl) rc = rl;
+          if (!rc) rc = launch_resident<T>(ctx, mask, rhs, x, r, p, Ap, st, (i - 1) * replace_every, replace_every);
         },
         out);
+    if (rc && gi >= 0) {  // no graph of a launch that was refused
+      cudaGraphExecDestroy(ctx->graphs[gi].exec);
+      ctx->graphs.erase(ctx->graphs.begin() + gi);
+    }
     return rc ? -1 : gi;
   }
   return capture_chunk(
@@ -777,9 +780,18 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
                   DevState *hst, int replace_every, bool confirm, bool rr, int *iters_out) {
   // resident iterations (grids that fit the chip): one kernel a checkpoint, so
   // a graph holds four checkpoints; past the end of a solve a kernel takes ~2 us
-  const bool resident = bbpp_persist_ok(ctx, (int)sizeof(T));
-  const int chunk = resident ? 4 * replace_every : ((replace_every % 2 == 0) ? replace_every : 2 * replace_every);
+  bool resident = bbpp_persist_ok(ctx, (int)sizeof(T));
+  const int single_chunk = (replace_every % 2 == 0) ? replace_every : 2 * replace_every;
+  int chunk = resident ? 4 * replace_every : single_chunk;
   if (resident && bbpp_persist_begin(ctx)) return BBPP_CUDA_ERROR;
+  // a cooperative launch that is refused (fewer SMs than the device reports): the solve, at whose state nothing
+  // has touched, and the context's later ones go on kernel by kernel
+  auto refused = [&](cudaError_t e) {
+    if (!resident || !bbpp_persist_refused(ctx, (int)sizeof(T), e)) return false;
+    resident = false;
+    chunk = single_chunk;
+    return true;
+  };
   // q = completed iterations, read back from the device
   CK(cudaMemcpyAsync(hst, st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -799,8 +811,13 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
     if (q % chunk == 0 && !ctx->profiling) {
       cudaGraphExec_t exec;
       gi = get_chunk_graph<T>(ctx, mask, rhs, x, r, p, Ap, st, chunk, replace_every, rr, resident, &exec);
-      if (gi < 0) return BBPP_CUDA_ERROR;
-      CK(cudaGraphLaunch(exec, ctx->stream));
+      if (gi < 0) {
+        if (refused(cudaSuccess)) continue;
+        return BBPP_CUDA_ERROR;
+      }
+      const cudaError_t e = cudaGraphLaunch(exec, ctx->stream);
+      if (refused(e)) continue;
+      CK(e);
       ctx->launches += ctx->graphs[gi].kernels;
     } else if (q % chunk == 0) {
       // profiling: the same chunk as direct launches enqueued back to back,
@@ -815,6 +832,7 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
       CK(cudaGetLastError());
     } else if (resident) {
       const int rl = launch_resident<T>(ctx, mask, rhs, x, r, p, Ap, st, q, replace_every);
+      if (rl && refused(cudaSuccess)) continue;
       if (rl) return rl;
       ctx->launches += 4;
       CK(cudaGetLastError());
@@ -1318,7 +1336,7 @@ extern "C" int bbpp_rhs_div(bbpp_ctx *ctx, double rho_f, double dt, const double
 extern "C" int bbpp_debug_wait(bbpp_ctx *ctx, long long wait_ns, int inject) {
   if (!ctx || wait_ns < 0) return BBPP_BAD_ARG;
   ctx->wait_ns = wait_ns;
-  ctx->inject = inject == INJECT_LAST_WAIT ? inject : (inject ? INJECT_COPIES : 0);
+  ctx->inject = inject >= INJECT_LAST_WAIT && inject <= INJECT_REFUSED ? inject : (inject ? INJECT_COPIES : 0);
   return 0;
 }
 

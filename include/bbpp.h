@@ -315,7 +315,8 @@ const char *bbpp_version(void);
  * waits (wait_ns > 0; 0 restores one second) and, with inject, make the next solves' waits run out, so that
  * they return BBPP_WAIT_TIMEOUT.  1: the kernels of FP32 solves leave one plane's copies unissued in a CTA
  * (the resident iteration an exchange).  2: the last CTA of the resident iteration (FP32 and FP64) takes the
- * wait that ends a solve for run out.  Nothing faults or hangs; the context stays usable. */
+ * wait that ends a solve for run out.  3: the resident iteration's launch is taken for refused (the solve goes
+ * on kernel by kernel, as do the context's later ones).  Nothing faults or hangs; the context stays usable. */
 int bbpp_debug_wait(bbpp_ctx *ctx, long long wait_ns, int inject);
 /* Select the GPU for this host thread's later contexts and buffers (one process per GPU; no counterpart in
  * the reference, whose ranks each own one GPU through cudaSetDevice in its start-up code). */

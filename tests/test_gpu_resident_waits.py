@@ -8,7 +8,7 @@ import bbpp
 from bbpp import problems
 
 pytestmark = pytest.mark.gpu
-LAST_WAIT = 2
+LAST_WAIT, REFUSED = 2, 3
 
 
 def problem(dims, bc, seed=3):
@@ -41,3 +41,26 @@ def test_a_wait_that_ran_out_is_not_overwritten(bbpp_lib, precision, dims):
     assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
     x, rep = s.solve_host(b, mask, tol=1e-8, precision=precision)
     assert rep.status == bbpp.CONVERGED and rep.true_rel <= 1.01e-8
+
+
+@pytest.mark.parametrize("precision,ir_mode", [(bbpp.FP64, 0), (bbpp.FP32_IR, bbpp.IR_RELIABLE),
+                                               (bbpp.FP32_IR, bbpp.IR_RESTART)])
+def test_a_refused_launch_falls_back(bbpp_lib, monkeypatch, precision, ir_mode):
+    """The cooperative launch is refused (the host's fake of the error): the solve
+    takes the kernels of single iterations, and the context's later solves those of a
+    context without the resident form, to the same bits."""
+    g, mask, b = problem((48, 40, 30), "ppn")
+    kw = dict(tol=1e-9, precision=precision, ir_mode=ir_mode)
+    s = bbpp.Solver(g)
+    L = bbpp.lib()
+    assert L.bbpp_debug_wait(s.handle, 0, REFUSED) == 0
+    x, rep = s.solve_host(b, mask, **kw)
+    assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
+    x1, rep1 = s.solve_host(b, mask, **kw)
+    monkeypatch.setenv("BBPP_PERSIST", "0")
+    later, _ = bbpp.Solver(g).solve_host(b, mask, **kw)
+    monkeypatch.setenv("BBPP_PAIR", "0")
+    first, rep0 = bbpp.Solver(g).solve_host(b, mask, **kw)
+    assert rep.status == rep1.status == bbpp.CONVERGED
+    assert rep.iters == rep0.iters and np.array_equal(x, first)
+    assert np.array_equal(x1, later)

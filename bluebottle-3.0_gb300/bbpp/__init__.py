@@ -318,7 +318,7 @@ class Solver:
         _check(lib().bbpp_set_profiling(self.handle, 1 if on else 0))
 
     def set_fused(self, on):
-        """FP32 reliable-update iterations as one fused kernel (True) or two."""
+        """Ask for FP32 reliable-update iterations as one fused kernel (True) or two."""
         _check(lib().bbpp_set_fused(self.handle, 1 if on else 0))
 
     def set_ff_resid(self, on):

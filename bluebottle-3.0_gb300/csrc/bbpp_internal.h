@@ -97,7 +97,9 @@ struct bbpp_ctx {
   bool pdl = false;               // iteration kernels launch with a programmatic dependency
   bool rev_update = true;         // the update kernel walks the search kernel's planes in reverse
   bool l2hint = true;             // FP32 iteration: mask evict_last in L2, p / Ap / x evict_first
-  bool fused = true;              // FP32 reliable-update solves: one fused kernel per iteration
+  // FP32 reliable-update solves: -1 the measured choice (resident iteration, pairs), 0 a search and an update
+  // kernel per iteration, 1 one fused kernel per iteration where the tensor-map kernels take the grid
+  int fused = -1;
   bool ff_resid = false;          // FP64 x -> FP32 r residuals in float-float arithmetic (else FP64)
   int inject = 0;                 // test hook of bbpp_debug_wait (see DevState::inject)
   long long wait_ns = 0;          // bound of device-side waits (0: one second)
@@ -219,6 +221,7 @@ int bbpp_pcg_loop_pair(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, flo
 void bbpp_persist_init(bbpp_ctx *ctx);
 void bbpp_persist_free(bbpp_ctx *ctx);
 bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem);
+bool bbpp_one_step(const bbpp_ctx *ctx);  // a one-iteration FP32 form was asked for
 int bbpp_persist_begin(bbpp_ctx *ctx);
 bool bbpp_persist_refused(bbpp_ctx *ctx, int elem, cudaError_t e);
 template <typename T>

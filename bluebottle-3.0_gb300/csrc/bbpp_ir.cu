@@ -86,8 +86,8 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   // 128^3 (2.1M) 17.0 and 26.1, 144^3 (3.0M) 22.1 and 29.4, 160^3 (4.1M) 28.2 and
   // 35.0 (walls 35.9 and 40.8), 168^3 (4.7M) 43.3 and 36.3, 176^3 (5.5M) 52.6 and 40.8.
   bool resident = bbpp_persist_ok(ctx, 4);
-  const bool pair =
-      ctx->fused && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 && (!resident || n > 4200000);
+  const bool pair = !bbpp_one_step(ctx) && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 &&
+                    (!resident || n > 4200000);
   if (pair) resident = false;
   hst->zform = pair ? 1 : 0;
   CK(cudaMemcpyAsync(st, hst, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
@@ -98,7 +98,7 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   bbpp_set_reliable(x, rhs);
   float *const p[2] = {b->p[0], b->p[1]};
   int it = 0;
-  bool fused = ctx->fused && bbpp_tma_fused_ok(ctx) && !resident && !pair;
+  bool fused = ctx->fused != 0 && bbpp_tma_fused_ok(ctx) && !resident && !pair;
   if (pair && !b->rd2) CK(cudaMalloc(&b->rd2, sizeof(float) * n));
   if (fused && !b->Ap2) {
     cudaFree(b->rd2);

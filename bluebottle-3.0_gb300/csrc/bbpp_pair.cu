@@ -773,9 +773,6 @@ void bbpp_pair_init(bbpp_ctx *ctx) {
   ctx->pair = t;
   const char *e = getenv("BBPP_PAIR");
   if (e && e[0] == '0') return;
-  // the warp-specialised fused kernel is asked for by its own variable
-  const char *ws = getenv("BBPP_FUSED_WS");
-  if (ws && atoi(ws) != 0) return;
   const GeoL &G = ctx->GL;
   if (G.nx % 4 != 0 || G.nx > 1024) return;
   const int nxv = G.nx / 4;

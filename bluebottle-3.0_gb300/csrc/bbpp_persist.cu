@@ -1127,10 +1127,7 @@ void bbpp_persist_init(bbpp_ctx *ctx) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   if (!coop) return;
   const int most = std::min(ctx->sms, kMaxCtas);
-  // the warp-specialised fused kernel is asked for by its own variable
-  const char *ws = getenv("BBPP_FUSED_WS");
-  const int k0 = ws && atoi(ws) != 0 ? 1 : 0;
-  for (int k = k0; k < 2; k++) {
+  for (int k = 0; k < 2; k++) {
     const int elem = k ? 8 : 4;
     Boxes &B = t->box[k];
     t->nth[k] = (ctx->GL.n + most - 1) / most <= 512 ? 256 : 512;
@@ -1178,8 +1175,11 @@ void bbpp_persist_free(bbpp_ctx *ctx) {
   ctx->persist = nullptr;
 }
 
+bool bbpp_one_step(const bbpp_ctx *ctx) { return ctx->fused == 0 || (ctx->fused == 1 && bbpp_tma_fused_ok(ctx)); }
+
 // Profiling times kernels one by one, so it runs the kernels of one iteration.
 bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem) {
+  if (elem == 4 && bbpp_one_step(ctx)) return false;
   return ctx->persist && ctx->persist->ok[elem == 8 ? 1 : 0] && !ctx->profiling;
 }
 

@@ -311,9 +311,11 @@ extern "C" int bbpp_create(const bbpp_grid *g, bbpp_ctx **out) {
     // persisting-L2 set-aside, is slower
     const char *lh = getenv("BBPP_L2HINT");
     ctx->l2hint = !(lh && lh[0] == '0');
-    // one fused kernel per FP32 iteration (BBPP_FUSED=0: search and update kernels)
+    // a form of the FP32 iteration asked for (BBPP_FUSED=1: one fused kernel, 0: search and update kernels;
+    // BBPP_FUSED_WS: a fused kernel, 1 the warp-specialised one)
     const char *fu = getenv("BBPP_FUSED");
-    ctx->fused = !(fu && fu[0] == '0');
+    if (fu && fu[0]) ctx->fused = fu[0] != '0';
+    else if (getenv("BBPP_FUSED_WS")) ctx->fused = 1;
     // residuals of FP64 x into FP32 r: FP64 arithmetic, the outer residual of
     // the mixed-precision method; BBPP_FF_RESID=1 selects float-float
     // arithmetic on the FP32 pipe (~48 bits; measured 0.2 ms per C3 solve)
@@ -1709,7 +1711,7 @@ void bbpp_rec_collect(bbpp_ctx *ctx, std::vector<KEv> &evs, int iters_done, bool
 
 extern "C" int bbpp_set_fused(bbpp_ctx *ctx, int on) {
   if (!ctx || (on != 0 && on != 1)) return BBPP_BAD_ARG;
-  ctx->fused = on == 1;
+  ctx->fused = on;
   return 0;
 }
 

@@ -232,10 +232,12 @@ int bbpp_kernel_stats(bbpp_ctx *ctx, bbpp_kstat *out, int max, int *n);
  * counters.  Kernels are timed one by one, so grids whose iterations run inside
  * one launch (csrc/bbpp_persist.cu) take the kernels of single iterations. */
 int bbpp_set_profiling(bbpp_ctx *ctx, int on);
-/* The FP32 iteration of reliable-update solves on grids that do not fit the
- * chip: 1 = pairs of iterations in two kernels (rows of a multiple of four
- * cells up to 1024; the default), 0 = a search kernel and an update kernel per
- * iteration. */
+/* Ask for a form of the FP32 iteration of reliable-update solves: 1 = one
+ * fused kernel per iteration where the tensor-map kernels take the grid (the
+ * library's choice elsewhere), 0 = a search kernel and an update kernel.  A
+ * context that is not asked takes the fastest: the resident iteration on grids
+ * that fit the chip, pairs of iterations in two kernels on larger ones with
+ * rows of a multiple of four cells up to 1024, else these two. */
 int bbpp_set_fused(bbpp_ctx *ctx, int on);
 /* The outer residuals of the reliable updates (FP64 x into the FP32
  * residual): 0 = FP64 arithmetic (the default), 1 = float-float arithmetic on

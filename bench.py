@@ -33,7 +33,7 @@ WORKLOAD = ("C3: 256^3 cells, periodic x/y + Neumann z, 1000 spheres r=6 cells, 
 # summaries sit with the other profiles): kernel kind -> bytes
 NCU_TRAFFIC = {"search_spmv_f32": 226.697984e6 + 150.230784e6, "search_spmv": 436.172800e6 + 366.177536e6,
                "update_f32": 134.251008e6 + 20.922112e6, "update": 268.485376e6 + 92.526592e6,
-               "fused_f32": 230.443520e6 + 147.042304e6, "dots_f32": 162.937088e6 + 2.969856e6}
+               "pair_f32": 230.443520e6 + 147.042304e6, "dots_f32": 162.937088e6 + 2.969856e6}
 
 
 # FP64-pipe thread instructions per cell per launch of the plain FP64 kernels on

@@ -39,7 +39,7 @@ struct KEv {
 };
 
 enum KernelKind { KK_SEARCH_SPMV = 0, KK_UPDATE, KK_AXPY, KK_RESID, KK_SEARCH_SPMV_F32, KK_UPDATE_F32,
-                  KK_AXPY_F32, KK_RESID_F32, KK_FUSED_F32, KK_DOTS_F32, KK_COUNT };
+                  KK_AXPY_F32, KK_RESID_F32, KK_FUSED_F32, KK_DOTS_F32, KK_PAIR_F32, KK_COUNT };
 
 struct GraphCache {
   GraphKey key;

@@ -996,7 +996,7 @@ static void launch_pair(bbpp_ctx *ctx, const uint8_t *mask, float *x, float *con
   bbpp_rec_begin(ctx, KK_DOTS_F32, 8.0 + (mask ? 1 : 0));
   bbpp_pair_launch(ctx, false, mask, z[i], p[i], nullptr, nullptr, nullptr, st, replace_every);
   bbpp_rec_end(ctx);
-  bbpp_rec_begin(ctx, KK_FUSED_F32, 24.0 + (mask ? 1 : 0));
+  bbpp_rec_begin(ctx, KK_PAIR_F32, 24.0 + (mask ? 1 : 0));
   bbpp_pair_launch(ctx, true, mask, z[i], p[i], z[o], p[o], x, st, replace_every);
   bbpp_rec_end(ctx);
 }
@@ -1664,7 +1664,7 @@ extern "C" int bbpp_stream_mix_rate(long long cells, double *bytes_per_s) {
 
 // ----------------------------------------------------------- kernel stats --
 static const char *kk_name[KK_COUNT] = {"search_spmv", "update", "axpy_x", "resid", "search_spmv_f32",
-                                        "update_f32", "axpy_x_f32", "resid_f32", "fused_f32", "dots_f32"};
+                                        "update_f32", "axpy_x_f32", "resid_f32", "fused_f32", "dots_f32", "pair_f32"};
 
 void bbpp_rec_begin(bbpp_ctx *ctx, int kind, double bytes_per_cell) {
   if (!ctx->rec) return;

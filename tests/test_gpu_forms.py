@@ -9,7 +9,7 @@ from bbpp import problems
 
 pytestmark = pytest.mark.gpu
 
-FORMS = {"default": {"fused_f32", "dots_f32"}, "fused": {"fused_f32"}, "two": {"search_spmv_f32", "update_f32"},
+FORMS = {"default": {"pair_f32", "dots_f32"}, "fused": {"fused_f32"}, "two": {"search_spmv_f32", "update_f32"},
          "ws0": {"fused_f32"}, "ws1": {"fused_f32"}}
 
 

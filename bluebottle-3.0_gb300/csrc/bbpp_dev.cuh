@@ -39,6 +39,7 @@ enum Inject : int {
   INJECT_COPIES = 1,     // FP32: the first CTA leaves one plane's copies out (the resident one's last CTA an exchange)
   INJECT_LAST_WAIT = 2,  // resident: the last CTA takes its last wait for run out
   INJECT_REFUSED = 3,    // resident: the host takes the launch for refused
+  INJECT_NO_MEMORY = 4,  // FP32: no memory for the vectors that only pairs and the fused iteration need
 };
 
 // Device-resident scalar state of one PCG solve.

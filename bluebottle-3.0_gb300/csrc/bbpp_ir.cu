@@ -57,6 +57,15 @@ __global__ void k_add_correction(const Geo G, double *__restrict__ x, const floa
 
 static int ensure_ir(bbpp_ctx *ctx);
 
+// a vector that only some forms of the iteration need: is it there?
+static bool extra(bbpp_ctx *ctx, float **p) {
+  if (*p) return true;
+  if (ctx->inject != INJECT_NO_MEMORY && cudaMalloc(p, sizeof(float) * (size_t)ctx->G.n) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
 // Reliable-update form: one FP32 PCG on L d = S rhs - L x; every residual
 // replacement (and the confirmation of a recursive convergence) adds d into x
 // in FP64, zeroes d and recomputes the residual from x in FP64.  The search
@@ -86,9 +95,13 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   // 128^3 (2.1M) 17.0 and 26.1, 144^3 (3.0M) 22.1 and 29.4, 160^3 (4.1M) 28.2 and
   // 35.0 (walls 35.9 and 40.8), 168^3 (4.7M) 43.3 and 36.3, 176^3 (5.5M) 52.6 and 40.8.
   bool resident = bbpp_persist_ok(ctx, 4);
-  const bool pair = !bbpp_one_step(ctx) && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 &&
-                    (!resident || n > 4200000);
+  bool pair = !bbpp_one_step(ctx) && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 && (!resident || n > 4200000);
+  // a second z for the pairs, a second r and Ap for the fused iteration; without the memory the solve takes a
+  // form that needs less
+  if (pair) pair = extra(ctx, &b->rd2);
   if (pair) resident = false;
+  bool fused = ctx->fused != 0 && bbpp_tma_fused_ok(ctx) && !resident && !pair;
+  if (fused) fused = extra(ctx, &b->rd2) && extra(ctx, &b->Ap2);
   hst->zform = pair ? 1 : 0;
   CK(cudaMemcpyAsync(st, hst, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(b->d, 0, sizeof(float) * n, ctx->stream));
@@ -98,14 +111,6 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   bbpp_set_reliable(x, rhs);
   float *const p[2] = {b->p[0], b->p[1]};
   int it = 0;
-  bool fused = ctx->fused != 0 && bbpp_tma_fused_ok(ctx) && !resident && !pair;
-  if (pair && !b->rd2) CK(cudaMalloc(&b->rd2, sizeof(float) * n));
-  if (fused && !b->Ap2) {
-    cudaFree(b->rd2);
-    b->rd2 = nullptr;
-    CK(cudaMalloc(&b->rd2, sizeof(float) * n));
-    CK(cudaMalloc(&b->Ap2, sizeof(float) * n));
-  }
   float *const rs[2] = {b->rd, b->rd2}, *const as[2] = {b->Ap, b->Ap2};
   if (fused) fused = bbpp_tma_fused_maps(ctx, rs, as, p);
   if (pair)

@@ -53,3 +53,29 @@ def test_a_form_asked_for_is_not_the_default(bbpp_lib, monkeypatch, form):
     x, rep = s.solve_host(rhs, mask, tol=1e-8, precision=bbpp.FP32_IR)
     y, rep2 = make(monkeypatch, "default")[0].solve_host(rhs, mask, tol=1e-8, precision=bbpp.FP32_IR)
     assert not np.array_equal(x, y) and np.abs(x - y).max() <= 1e-5 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("form,dims", [("pair", (64, 45, 30)), ("pair", (64, 64, 64)), ("fused", (64, 64, 64))])
+def test_no_memory_for_a_form(bbpp_lib, monkeypatch, form, dims):
+    """The vectors that only the pairs or the fused iteration need cannot be had (the
+    host's fake of the failing call): the solve takes the search and update kernels,
+    which need none, to the same bits; with memory again, the form itself."""
+    monkeypatch.setenv("BBPP_PERSIST", "0")
+    if form == "fused":
+        monkeypatch.setenv("BBPP_PAIR", "0")
+    nx, ny, nz = dims
+    g = bbpp.Grid.make(nx, ny, nz, 1.0 / nx, 1.0 / ny, 1.0 / nz, problems.bc_tuple("ppn"))
+    rng = np.random.default_rng(1)
+    b = rng.uniform(-1, 1, g.shape)
+    b -= b.mean()
+    kw = dict(tol=1e-8, precision=bbpp.FP32_IR)
+    s, s2 = bbpp.Solver(g), bbpp.Solver(g)
+    s2.set_fused(False)
+    x2, _ = s2.solve_host(b, None, **kw)
+    L = bbpp.lib()
+    assert L.bbpp_debug_wait(s.handle, 0, 4) == 0
+    x, rep = s.solve_host(b, None, **kw)
+    assert rep.status == bbpp.CONVERGED and np.array_equal(x, x2)
+    assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
+    x, rep = s.solve_host(b, None, **kw)
+    assert rep.status == bbpp.CONVERGED and not np.array_equal(x, x2)

@@ -175,7 +175,10 @@ __device__ __forceinline__ unsigned int ld_u32_pol(const void *a, unsigned long 
 // instruction on the FP64 pipe (1/64 of the FP32 rate).  Zero keeps its sign;
 // subnormal inputs (never produced by the solver's vectors in practice) take
 // the conversion instruction.
-__device__ __forceinline__ double widen_f32(float f) {
+__host__ __device__ __forceinline__ double widen_f32(float f) {
+#ifndef __CUDA_ARCH__
+  return (double)f;
+#else
   const unsigned int u = __float_as_uint(f);
   const unsigned long long sign = (unsigned long long)(u & 0x80000000u) << 32;
   const unsigned int e32 = (u >> 23) & 0xffu;
@@ -183,6 +186,36 @@ __device__ __forceinline__ double widen_f32(float f) {
   if (e32 == 0) return frac ? (double)f : __longlong_as_double((long long)sign);
   if (e32 == 0xffu) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull | frac));
   return __longlong_as_double((long long)(sign | ((unsigned long long)(e32 - 127u + 1023u) << 52) | frac));
+#endif
+}
+
+// v[lane] + v[lane + 32] + ... (below n) to FP64's quality with FP32 operations: FP64
+// adds of one value a thread would hold the FP64 pipe 16 cycles a warp each.  Three
+// floats carry the sum (two-sums, Knuth; in cascade, Ogita, Rump, Oishi 2005): its
+// error is 2^-53 of it and (n / 32)^2 2^-72 of the values' magnitudes, below that of
+// n / 32 FP64 adds.  What FP32 cannot hold (a sum out of its range, infinities, NaN)
+// is added in FP64.
+__host__ __device__ __noinline__ static double sum_floats_fp64(const float *v, int n, int lane) {
+  double a = 0.0;
+  for (int e = lane; e < n; e += 32) a += (double)v[e];
+  return a;
+}
+__host__ __device__ __forceinline__ float two_sum(float &a, float b) {  // a += b; returns what that lost
+#ifdef __CUDA_ARCH__
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+#else
+  const float s = a + b, t = s - a, e = (a - (s - t)) + (b - t);
+#endif
+  a = s;
+  return e;
+}
+__host__ __device__ __forceinline__ double sum_floats(const float *v, int n, int lane) {
+  float hi = v[lane], mid = 0.f, lo = 0.f;
+  for (int e = lane + 32; e < n; e += 32) lo += two_sum(mid, two_sum(hi, v[e]));
+  const float t = hi + mid + lo;
+  if (!(t >= -3.402823466e38f && t <= 3.402823466e38f)) return sum_floats_fp64(v, n, lane);
+  return widen_f32(hi) + (widen_f32(mid) + widen_f32(lo));
 }
 
 __device__ __forceinline__ unsigned int fdiv(unsigned int n, unsigned long long m) {

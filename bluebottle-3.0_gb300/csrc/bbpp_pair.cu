@@ -118,16 +118,6 @@ __device__ __forceinline__ float4 fma4(const float2 a, const float4 b, const flo
   return join(__ffma2_rn(a, lo2(b), lo2(c)), __ffma2_rn(a, hi2(b), hi2(c)));
 }
 
-// Neumaier-style sum of floats as an unevaluated pair (two-sum, Knuth)
-struct Pairf {
-  float hi, lo;
-};
-__device__ __forceinline__ void add_to(Pairf &a, float v) {
-  const float s = __fadd_rn(a.hi, v), b = __fsub_rn(s, a.hi);
-  a.lo = __fadd_rn(a.lo, __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, b)), __fsub_rn(v, b)));
-  a.hi = s;
-}
-
 }  // namespace
 
 namespace bbpp {
@@ -708,9 +698,8 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
     return;
   }
   if (STEP) return;
-  // The CTA's sums: per thread in FP32, summed across threads as unevaluated
-  // pairs of floats (48 bits; FP64 adds for 512 threads x 11 products would take
-  // the FP64 pipe 2.5 us a launch), in FP64 from warps on.
+  // The CTA's sums: per thread in FP32, across threads by sum_floats (FP64 adds for
+  // 512 threads x 11 products would take the FP64 pipe 2.5 us a launch).
   float *sv = reinterpret_cast<float *>(smem_raw);  // [NDOT][threads]
   const int nth = blockDim.x;
 #pragma unroll
@@ -718,9 +707,7 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   __syncthreads();
   const unsigned int nb = gridDim.x * gridDim.y, bid = blockIdx.x + gridDim.x * blockIdx.y;
   for (int k = tid >> 5; k < NDOT; k += nth >> 5) {  // a warp a product
-    Pairf a = {0.f, 0.f};
-    for (int e = lane; e < nth; e += 32) add_to(a, sv[k * nth + e]);
-    const double v = warp_sum(widen_f32(a.hi) + widen_f32(a.lo));
+    const double v = warp_sum(sum_floats(sv + k * nth, nth, lane));
     if (lane == 0) partials[(size_t)k * nb + bid] = v;
   }
   __threadfence();

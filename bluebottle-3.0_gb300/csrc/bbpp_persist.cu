@@ -213,21 +213,8 @@ __device__ __forceinline__ void exchange(const double (&v)[NV], double (&tot)[NV
 }
 
 // The same for the NV products of a one-exchange iteration (NV <= 7), each summed by a
-// warp of its own: over the CTA's threads (FP32 partial sums as unevaluated pairs of
-// floats, 48 bits), then over the CTAs' slots, in fixed order.  Warp 7 counts the CTA
+// warp of its own: over the CTA's threads (sum_floats), then over the CTAs' slots, in fixed order.  Warp 7 counts the CTA
 // in, its earlier global writes before it, and waits.  Totals in s_tot.
-struct PairF {
-  float hi, lo;
-};
-__device__ __forceinline__ double sum_strided(const float *v, int n, int lane) {
-  PairF a = {v[lane], 0.f};
-  for (int e = lane + 32; e < n; e += 32) {  // two-sum (Knuth)
-    const float x = v[e], s = __fadd_rn(a.hi, x), b = __fsub_rn(s, a.hi);
-    a.lo = __fadd_rn(a.lo, __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
-    a.hi = s;
-  }
-  return widen_f32(a.hi) + widen_f32(a.lo);
-}
 template <int NV, int NTH>
 __device__ __forceinline__ void exchange_all(const float (&v)[NV], double *s_tot, bbpp_exchange *ex,
                                              Slot (*slots)[kMaxCtas], int nb, unsigned long long n,
@@ -241,7 +228,7 @@ __device__ __forceinline__ void exchange_all(const float (&v)[NV], double *s_tot
 #pragma unroll
     for (int q = q0; q < NV && q < q0 + 4; q++) s_part[(q - q0) * NTH + tid] = v[q];
     __syncthreads();
-    if (warp >= q0 && warp < q0 + 4 && warp < NV) a = warp_sum(sum_strided(s_part + (warp - q0) * NTH, NTH, lane));
+    if (warp >= q0 && warp < q0 + 4 && warp < NV) a = warp_sum(sum_floats(s_part + (warp - q0) * NTH, NTH, lane));
   }
   if (warp < NV) {
     if (lane == 0 && !silent) slot_put(&slots[warp][blockIdx.x], a, n);

@@ -314,9 +314,9 @@ __global__ void __launch_bounds__(NTH, 1) k_persist(const GeoL G, const Boxes B,
   const bool lag = !first && *(volatile int *)&st->dlag;
   const long long wl = *(volatile long long *)&st->wait_ns;
   const unsigned long long limit = wl > 0 ? (unsigned long long)wl : 1000000000ull;
-  // test hook (FP32 solves): the last CTA leaves its first exchange out
+  // test hooks, all of them in the last CTA
   const int inject = blockIdx.x == (unsigned)B.nb - 1u ? *(volatile int *)&st->inject : 0;
-  const bool silent0 = sizeof(T) == 4 && inject == INJECT_COPIES;
+  const bool silent0 = inject == INJECT_EXCHANGE || (sizeof(T) == 4 && inject == INJECT_COPIES);
   const int tid = threadIdx.x;
   if (tid < 27) s_inv[tid] = sizeof(T) == 8 ? (T)G.invL[tid] : (T)G.finvL[tid];
   if (tid < 27) s_dm1[tid] = (sizeof(T) == 8 ? (T)G.dL[tid] : (T)G.fdL[tid]) - T(1);

@@ -8,7 +8,7 @@ import bbpp
 from bbpp import problems
 
 pytestmark = pytest.mark.gpu
-LAST_WAIT, REFUSED = 2, 3
+LAST_WAIT, REFUSED, EXCHANGE = 2, 3, 5
 
 
 def problem(dims, bc, seed=3):
@@ -64,3 +64,42 @@ def test_a_refused_launch_falls_back(bbpp_lib, monkeypatch, precision, ir_mode):
     assert rep.status == rep1.status == bbpp.CONVERGED
     assert rep.iters == rep0.iters and np.array_equal(x, first)
     assert np.array_equal(x1, later)
+
+
+@pytest.mark.parametrize("precision", [bbpp.FP64, bbpp.FP32_IR])
+@pytest.mark.parametrize("dims", [(12, 9, 7), (40, 33, 29), (128, 100, 90)])
+def test_an_exchange_without_a_cta(bbpp_lib, precision, dims):
+    """Every CTA's wait gives up and returns, in FP64 as in FP32, and the next solve
+    starts from clean counts."""
+    g, mask, b = problem(dims, "pnp")
+    s = bbpp.Solver(g)
+    L = bbpp.lib()
+    for _ in range(2):
+        assert L.bbpp_debug_wait(s.handle, 2_000_000, EXCHANGE) == 0   # 2 ms
+        x, rep = s.solve_host(b, mask, tol=1e-8, precision=precision, ok=ANY)
+        assert rep.status == bbpp.WAIT_TIMEOUT
+        assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
+        x, rep = s.solve_host(b, mask, tol=1e-8, precision=precision)
+        assert rep.status == bbpp.CONVERGED and rep.true_rel <= 1.01e-8
+
+
+@pytest.mark.parametrize("precision", [bbpp.FP64, bbpp.FP32_IR])
+@pytest.mark.parametrize("dims", [(48, 40, 36), (130, 120, 118), (160, 150, 140)])
+@pytest.mark.parametrize("max_iter", [5, 48, 49, 50, 63])
+def test_the_solution_of_an_unfinished_solve(bbpp_lib, monkeypatch, precision, dims, max_iter):
+    """The state that a launch leaves at an iteration limit, before, on and after a
+    checkpoint and with all of it, some or none in shared memory: the two-kernel
+    iteration's solution."""
+    if precision == bbpp.FP64 and dims[0] == 160:
+        pytest.skip("FP64 grids of this size are not resident")
+    g, mask, b = problem(dims, "ppn", 5)
+    kw = dict(tol=1e-14, precision=precision, max_iter=max_iter, ok=(bbpp.MAX_ITER,))
+    x, rep = bbpp.Solver(g).solve_host(b, mask, **kw)
+    monkeypatch.setenv("BBPP_PERSIST", "0")
+    s = bbpp.Solver(g)
+    s.set_fused(False)
+    y, rep2 = s.solve_host(b, mask, **kw)
+    assert rep.status == rep2.status == bbpp.MAX_ITER and rep.iters == rep2.iters == max_iter + 1
+    # rounding (2^-53, 2^-24) times the condition number, below (2 n / pi)^2 = 1e4 for 160 cells
+    eps = 2.0 ** -53 if precision == bbpp.FP64 else 2.0 ** -24
+    assert np.abs(x - y).max() <= 1e4 * eps * np.abs(y).max()

@@ -550,22 +550,26 @@ __global__ void k_up_bwd(const bf16 *__restrict__ dout, int ldo, int off, int C,
   }
 }
 
-// g[v][c] (ld C) = dout[v][c] (ld C) * (out[v][off + c] > 0)   (ReLU backward)
-// g = dout where the layer's output is positive, else 0; db[c] += sum_v g[v][c].
-// Eight channels (16 bytes) a thread; a thread keeps its channels from voxel to
-// voxel, so the bias sums stay in registers.  One pass: the gate and the bias
-// gradient apart took 71 + 35 us for 16 channels of four 64^3 volumes.
+// ReLU backward: g = dout where the layer's output is positive, else 0 (g and dout
+// dense, C = 16, 32 or 64 channels), and sums of g over the voxels for db (k_bias_out).
+// Eight channels (16 bytes) a thread; a thread keeps its channels from voxel to voxel,
+// so the bias sums stay in registers.  One pass: the gate and the bias gradient apart
+// took 71 + 35 us for 16 channels of four 64^3 volumes.  The CTAs' sums meet in FP64:
+// FP32 atomics on db, up to kGateCtas of them a channel, had up to six times the error
+// of the two passes (now a tenth to a half of it).  kGateSums places a channel: on one,
+// the CTAs wait for each other's atomics (4 us a layer).
+constexpr int kGateCtas = 1216, kGateSums = 16;
 __global__ void __launch_bounds__(256) k_gate_bias(const bf16 *__restrict__ dout, const bf16 *__restrict__ out,
                                                    int ldo, int off, int C, long long nvox, bf16 *__restrict__ g,
-                                                   float *db) {
-  __shared__ float s[256][9];
-  const int parts = C / 8, part = threadIdx.x % parts, per = 256 / parts;  // C = 16, 32 or 64
+                                                   double *sum) {
+  __shared__ float s[8][64];
+  const int parts = C / 8, c8 = threadIdx.x % parts, per = 256 / parts;
   float a[8];
 #pragma unroll
   for (int q = 0; q < 8; q++) a[q] = 0.f;
   for (long long v = blockIdx.x * (long long)per + threadIdx.x / parts; v < nvox; v += (long long)gridDim.x * per) {
-    const uint4 du = *reinterpret_cast<const uint4 *>(dout + v * C + part * 8);
-    const uint4 ou = *reinterpret_cast<const uint4 *>(out + v * ldo + off + part * 8);
+    const uint4 du = *reinterpret_cast<const uint4 *>(dout + v * C + c8 * 8);
+    const uint4 ou = *reinterpret_cast<const uint4 *>(out + v * ldo + off + c8 * 8);
     float d[8], o[8];
     bf8_unpack(du, d);
     bf8_unpack(ou, o);
@@ -574,16 +578,40 @@ __global__ void __launch_bounds__(256) k_gate_bias(const bf16 *__restrict__ dout
       d[q] = o[q] > 0.f ? d[q] : 0.f;
       a[q] += d[q];
     }
-    *reinterpret_cast<uint4 *>(g + v * C + part * 8) = bf8_pack(d);
+    *reinterpret_cast<uint4 *>(g + v * C + c8 * 8) = bf8_pack(d);
   }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o = 16; o >= parts; o >>= 1) {
 #pragma unroll
-  for (int q = 0; q < 8; q++) s[threadIdx.x][q] = a[q];
+    for (int q = 0; q < 8; q++) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+  }
+  if (lane < parts) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) s[warp][lane * 8 + q] = a[q];
+  }
   __syncthreads();
   if (threadIdx.x < (unsigned)C) {
-    float t = 0.f;
-    for (int i = threadIdx.x / 8; i < 256; i += parts) t += s[i][threadIdx.x % 8];
-    atomicAdd(&db[threadIdx.x], t);
+    float t[8];
+#pragma unroll
+    for (int w = 0; w < 8; w++) t[w] = s[w][threadIdx.x];
+    atomicAdd(&sum[blockIdx.x % kGateSums * 64 + threadIdx.x],
+              (double)(((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]))));
   }
+}
+
+// db[c] += the sums of k_gate_bias, a layer a CTA
+static_assert(kGateSums == 16, "four places in each quarter");
+struct BiasOffsets {
+  int off[5], n[5];
+};
+__global__ void __launch_bounds__(256) k_bias_out(const double *__restrict__ sums, const BiasOffsets L, float *grads) {
+  __shared__ double s[4][64];
+  const int c = threadIdx.x & 63, part = threadIdx.x >> 6;  // a quarter of the places
+  const double *v = sums + (blockIdx.x * kGateSums + part * (kGateSums / 4)) * 64 + c;
+  s[part][c] = (v[0] + v[64]) + (v[128] + v[192]);
+  __syncthreads();
+  if (part == 0 && c < L.n[blockIdx.x])
+    grads[L.off[blockIdx.x] + c] += (float)((s[0][c] + s[1][c]) + (s[2][c] + s[3][c]));
 }
 
 // OUT[v] = D1[v] . w + b   (FP32)
@@ -882,6 +910,7 @@ struct bbpp_net {
        *D1 = nullptr;
   float *OUT = nullptr, *dOUT = nullptr, *scales = nullptr;
   double *sums = nullptr, *lossd = nullptr;
+  double *bsum = nullptr;  // bias gradients: the CTAs' sums of each layer
   bf16 *dD1 = nullptr, *G = nullptr, *dCAT1 = nullptr, *dD2 = nullptr, *dCAT2 = nullptr, *dE3 = nullptr,
        *dP2 = nullptr, *dE2 = nullptr, *dP1 = nullptr, *dE1 = nullptr;
   cudaStream_t stream = nullptr;
@@ -896,12 +925,14 @@ static unsigned long long g_net_uid = 0;
 static void free_work(bbpp_net *n) {
   n->gen++;
   void *ptrs[] = {n->X0, n->CAT1, n->P1, n->CAT2, n->P2, n->E3, n->D2, n->D1, n->OUT, n->dOUT, n->scales, n->sums,
-                  n->lossd, n->dD1, n->G, n->dCAT1, n->dD2, n->dCAT2, n->dE3, n->dP2, n->dE2, n->dP1, n->dE1};
+                  n->lossd, n->dD1, n->G, n->dCAT1, n->dD2, n->dCAT2, n->dE3, n->dP2, n->dE2, n->dP1, n->dE1,
+                  n->bsum};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   n->X0 = n->CAT1 = n->P1 = n->CAT2 = n->P2 = n->E3 = n->D2 = n->D1 = nullptr;
   n->OUT = n->dOUT = n->scales = nullptr;
   n->sums = n->lossd = nullptr;
+  n->bsum = nullptr;
   n->dD1 = n->G = n->dCAT1 = n->dD2 = n->dCAT2 = n->dE3 = n->dP2 = n->dE2 = n->dP1 = n->dE1 = nullptr;
   n->wx = n->wy = n->wz = n->wb = 0;
 }
@@ -935,6 +966,7 @@ static int ensure_work(bbpp_net *n, int nx, int ny, int nz, int nb, bool grads) 
     NCK(cudaMalloc(&n->dE2, V2 * 32 * B));
     NCK(cudaMalloc(&n->dP1, V2 * 16 * B));
     NCK(cudaMalloc(&n->dE1, V * 16 * B));
+    NCK(cudaMalloc(&n->bsum, NLAYER * 64 * kGateSums * sizeof(double)));
   }
   n->wx = nx;
   n->wy = ny;
@@ -1044,10 +1076,12 @@ static int backward(bbpp_net *n, int nx, int ny, int nz, int nb) {
   const ConvLayer *L = n->L;
   float *G32 = n->g;
   cudaError_t e;
+  NCK(cudaMemsetAsync(n->bsum, 0, NLAYER * 64 * kGateSums * sizeof(double), s));
   k_head_bwd<<<nblocks(V), 256, 0, s>>>(n->dOUT, n->D1, n->w + n->head_w, V, n->dD1, G32 + n->head_w,
                                         G32 + n->head_b);
   // D1 = relu(conv(CAT1))
-  k_gate_bias<<<std::min(nblocks(V * 2), 1216), 256, 0, s>>>(n->dD1, n->D1, 16, 0, 16, V, n->G, G32 + L[4].boff);
+  k_gate_bias<<<std::min(nblocks(V * 2), kGateCtas), 256, 0, s>>>(n->dD1, n->D1, 16, 0, 16, V, n->G,
+                                                                  n->bsum + 4 * 64 * kGateSums);
   e = conv_wgrad(48, 16, wargs(nx, ny, nz, nb, n->CAT1, 48, 0, n->G, 16, G32 + L[4].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(16, 48, cargs(n, nx, ny, nz, nb, n->G, 16, 0, n->wt16 + L[4].woff, nullptr, n->dCAT1, 48, 0, 0), s);
@@ -1055,7 +1089,8 @@ static int backward(bbpp_net *n, int nx, int ny, int nz, int nb) {
   // CAT1[:, 0:32] = up(D2)
   k_up_bwd<<<nblocks(V2 * 32), 256, 0, s>>>(n->dCAT1, 48, 0, 32, nx, ny, nz, nb, n->dD2);
   // D2 = relu(conv(CAT2))
-  k_gate_bias<<<std::min(nblocks(V2 * 4), 1216), 256, 0, s>>>(n->dD2, n->D2, 32, 0, 32, V2, n->G, G32 + L[3].boff);
+  k_gate_bias<<<std::min(nblocks(V2 * 4), kGateCtas), 256, 0, s>>>(n->dD2, n->D2, 32, 0, 32, V2, n->G,
+                                                                  n->bsum + 3 * 64 * kGateSums);
   e = conv_wgrad(96, 32, wargs(hx, hy, hz, nb, n->CAT2, 96, 0, n->G, 32, G32 + L[3].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(32, 96, cargs(n, hx, hy, hz, nb, n->G, 32, 0, n->wt16 + L[3].woff, nullptr, n->dCAT2, 96, 0, 0), s);
@@ -1063,23 +1098,32 @@ static int backward(bbpp_net *n, int nx, int ny, int nz, int nb) {
   // CAT2[:, 0:64] = up(E3)
   k_up_bwd<<<nblocks(V4 * 64), 256, 0, s>>>(n->dCAT2, 96, 0, 64, hx, hy, hz, nb, n->dE3);
   // E3 = relu(conv(P2))
-  k_gate_bias<<<std::min(nblocks(V4 * 8), 1216), 256, 0, s>>>(n->dE3, n->E3, 64, 0, 64, V4, n->G, G32 + L[2].boff);
+  k_gate_bias<<<std::min(nblocks(V4 * 8), kGateCtas), 256, 0, s>>>(n->dE3, n->E3, 64, 0, 64, V4, n->G,
+                                                                  n->bsum + 2 * 64 * kGateSums);
   e = conv_wgrad(32, 64, wargs(qx, qy, qz, nb, n->P2, 32, 0, n->G, 64, G32 + L[2].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(64, 32, cargs(n, qx, qy, qz, nb, n->G, 64, 0, n->wt16 + L[2].woff, nullptr, n->dP2, 32, 0, 0), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   // E2 (in CAT2[:, 64:96]): skip gradient dCAT2[:, 64:96] + pool backward of dP2
   k_pool_bwd<<<nblocks(V2 * 32), 256, 0, s>>>(n->dP2, n->dCAT2, 96, 64, 32, hx, hy, hz, nb, n->dE2);
-  k_gate_bias<<<std::min(nblocks(V2 * 4), 1216), 256, 0, s>>>(n->dE2, n->CAT2, 96, 64, 32, V2, n->G, G32 + L[1].boff);
+  k_gate_bias<<<std::min(nblocks(V2 * 4), kGateCtas), 256, 0, s>>>(n->dE2, n->CAT2, 96, 64, 32, V2, n->G,
+                                                                  n->bsum + 1 * 64 * kGateSums);
   e = conv_wgrad(16, 32, wargs(hx, hy, hz, nb, n->P1, 16, 0, n->G, 32, G32 + L[1].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   e = conv_fwd(32, 16, cargs(n, hx, hy, hz, nb, n->G, 32, 0, n->wt16 + L[1].woff, nullptr, n->dP1, 16, 0, 0), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
   // E1 (in CAT1[:, 32:48]): skip gradient dCAT1[:, 32:48] + pool backward of dP1
   k_pool_bwd<<<nblocks(V * 16), 256, 0, s>>>(n->dP1, n->dCAT1, 48, 32, 16, nx, ny, nz, nb, n->dE1);
-  k_gate_bias<<<std::min(nblocks(V * 2), 1216), 256, 0, s>>>(n->dE1, n->CAT1, 48, 32, 16, V, n->G, G32 + L[0].boff);
+  k_gate_bias<<<std::min(nblocks(V * 2), kGateCtas), 256, 0, s>>>(n->dE1, n->CAT1, 48, 32, 16, V, n->G,
+                                                                  n->bsum + 0 * 64 * kGateSums);
   e = conv_wgrad(16, 16, wargs(nx, ny, nz, nb, n->X0, 16, 0, n->G, 16, G32 + L[0].woff), s);
   if (e != cudaSuccess) return BBPP_CUDA_ERROR;
+  BiasOffsets B;
+  for (int l = 0; l < NLAYER; l++) {
+    B.off[l] = L[l].boff;
+    B.n[l] = L[l].cout;
+  }
+  k_bias_out<<<NLAYER, 256, 0, s>>>(n->bsum, B, G32);
   NCK(cudaGetLastError());
   return 0;
 }

@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -312,23 +313,23 @@ cudaError_t conv_fwd(int cin, int cout, const ConvArgs &a, cudaStream_t s) {
 template <int CIN, int COUT>
 cudaError_t conv_wgrad_t(WgradArgs a, cudaStream_t s) {
   constexpr int smem = conv_wgrad_smem<CIN, COUT>();
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv3_wgrad<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
   const long long ntiles = (long long)((a.nx + CTX - 1) / CTX) * ((a.ny + CTY - 1) / CTY) *
                            ((a.nz + CTZ - 1) / CTZ) * a.nb;
   if (ntiles >= (1ll << 31)) return cudaErrorInvalidValue;
-  // one wave: every CTA adds its sums to dW once, so more CTAs are more atomics
-  static int wave = 0;
+  // one wave: every CTA adds its sums to dW once, so more CTAs are more atomics.  Asked of each device once (the
+  // shared memory cap is a device's too).
+  static std::atomic<int> waves[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int wave = dev < 64 ? waves[dev].load() : 0;
   if (!wave) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
+    cudaError_t e = cudaFuncSetAttribute(k_conv3_wgrad<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3_wgrad<CIN, COUT>, 256, smem);
     wave = std::max(1, sms) * std::max(1, per_sm);
+    if (dev < 64) waves[dev].store(wave);
   }
   constexpr int chunks = CIN / 16, groups = (27 + 8 * wgrad_taps<COUT>() - 1) / (8 * wgrad_taps<COUT>());
   // and more roundings: eight tiles a CTA at least, on small volumes

@@ -9,6 +9,7 @@
 // instantiated for float.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -83,7 +84,7 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   hst->tol2bb = o->tol * o->tol * (o->stop == 0 ? S : S * S);
   hst->tiny = 1e-16;
   hst->rep_d2 = o->ir_drop * o->ir_drop;
-  hst->rep_maxgap = 8 * o->replace_every;
+  hst->rep_maxgap = (int)std::min(8ll * o->replace_every, 1ll << 30);
   hst->max_iter = o->max_iter;
   hst->inject = ctx->inject;
   hst->wait_ns = ctx->wait_ns;

@@ -665,7 +665,7 @@ static void launch_iteration(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T
 template <typename T>
 static int launch_resident(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, T *const p[2], T *Ap,
                            DevState *st, int q, int replace_every) {
-  const int qc = (q / replace_every + 1) * replace_every;
+  const long long qc = (q / replace_every + 1ll) * replace_every;
   const int rc = bbpp_persist<T>(ctx, mask, r, p, Ap, x, st, replace_every);
   if (rc) return rc;  // nothing has run
   launch_update<T>(ctx, r, Ap, st, 1);
@@ -784,7 +784,8 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
   // a graph holds four checkpoints; past the end of a solve a kernel takes ~2 us
   bool resident = bbpp_persist_ok(ctx, (int)sizeof(T));
   const int single_chunk = (replace_every % 2 == 0) ? replace_every : 2 * replace_every;
-  int chunk = resident ? 4 * replace_every : single_chunk;
+  const int resident_chunk = replace_every <= (1 << 28) ? 4 * replace_every : replace_every;
+  int chunk = resident ? resident_chunk : single_chunk;
   if (resident && bbpp_persist_begin(ctx)) return BBPP_CUDA_ERROR;
   // a cooperative launch that is refused (fewer SMs than the device reports): the solve, at whose state nothing
   // has touched, and the context's later ones go on kernel by kernel
@@ -1183,12 +1184,17 @@ static int true_rel(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs, const
 
 // The solve without the final residual check: guess, solver, the device time
 // of both in rep->ms.  x is final when it returns (its stream has it in order).
-static int solve_core(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs, double *x, const bbpp_opts *o,
+static int solve_core(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs, double *x, const bbpp_opts *opts,
                       bbpp_report *rep) {
   memset(rep, 0, sizeof(*rep));
   if (!ctx || !rhs || !x) return rep->status = BBPP_BAD_ARG;
-  int rc = check_opts(o);
+  int rc = check_opts(opts);
   if (rc) return rep->status = rc;
+  // Checkpoints past the iteration limit are never met: one such spacing is as good as another, and the loops
+  // count and capture up to a checkpoint or several.
+  bbpp_opts lim = *opts;
+  lim.replace_every = (int)std::min<long long>(lim.replace_every, lim.max_iter + 2ll);
+  const bbpp_opts *o = &lim;
   ctx->launches = 0;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   bool zero_x = o->guess == BBPP_GUESS_ZERO;

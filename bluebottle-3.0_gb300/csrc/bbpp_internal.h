@@ -220,7 +220,7 @@ int bbpp_pcg_loop_pair(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, flo
 // iterations up to the next checkpoint in one resident kernel (bbpp_persist.cu)
 void bbpp_persist_init(bbpp_ctx *ctx);
 void bbpp_persist_free(bbpp_ctx *ctx);
-bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem);
+bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem, int replace_every);
 bool bbpp_one_step(const bbpp_ctx *ctx);  // a one-iteration FP32 form was asked for
 int bbpp_persist_begin(bbpp_ctx *ctx);
 bool bbpp_persist_refused(bbpp_ctx *ctx, int elem, cudaError_t e);

@@ -95,8 +95,14 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
   // the line is at 4.2M cells, us an iteration of a solve, resident and in pairs:
   // 128^3 (2.1M) 17.0 and 26.1, 144^3 (3.0M) 22.1 and 29.4, 160^3 (4.1M) 28.2 and
   // 35.0 (walls 35.9 and 40.8), 168^3 (4.7M) 43.3 and 36.3, 176^3 (5.5M) 52.6 and 40.8.
-  bool resident = bbpp_persist_ok(ctx, 4);
-  bool pair = !bbpp_one_step(ctx) && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 && (!resident || n > 4200000);
+  // With a checkpoint every iteration neither has more than one to do.  Where the
+  // tensor-map kernels take the grid one iteration at a time is faster then (ms a solve
+  // one by one and otherwise: 64^3 13.9 and 17.1, 128^3 27.8 and 34.8 resident; 256^3 88
+  // and 109 in pairs), elsewhere not: 100x76x60 27.7, resident 25.2, in pairs 20.8.
+  const bool one = bbpp_one_step(ctx), every = o->replace_every == 1;
+  bool resident = bbpp_persist_ok(ctx, 4, o->replace_every);
+  bool pair = !one && bbpp_pair_ok(ctx) && ((uintptr_t)mask & 3u) == 0 &&
+              (every ? !bbpp_tma_fused_ok(ctx) : !resident || n > 4200000);
   // a second z for the pairs, a second r and Ap for the fused iteration; without the memory the solve takes a
   // form that needs less
   if (pair) pair = extra(ctx, &b->rd2);

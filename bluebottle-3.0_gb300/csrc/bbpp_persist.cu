@@ -1164,9 +1164,12 @@ void bbpp_persist_free(bbpp_ctx *ctx) {
 
 bool bbpp_one_step(const bbpp_ctx *ctx) { return ctx->fused == 0 || (ctx->fused == 1 && bbpp_tma_fused_ok(ctx)); }
 
-// Profiling times kernels one by one, so it runs the kernels of one iteration.
-bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem) {
+// Profiling times kernels one by one, so it runs the kernels of one iteration.  FP32 with a checkpoint every
+// iteration: only small grids without the tensor-map kernels gain by a launch an iteration (ms a solve, resident and
+// one by one: 45x33x27 10.0 and 15.6, 90x75x58 31.4 and 35.4, 121x111x101 33.8 and 33.1).
+bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem, int replace_every) {
   if (elem == 4 && bbpp_one_step(ctx)) return false;
+  if (elem == 4 && replace_every == 1 && (bbpp_tma_fused_ok(ctx) || ctx->GL.n > 1 << 19)) return false;
   return ctx->persist && ctx->persist->ok[elem == 8 ? 1 : 0] && !ctx->profiling;
 }
 

@@ -782,7 +782,7 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
                   DevState *hst, int replace_every, bool confirm, bool rr, int *iters_out) {
   // resident iterations (grids that fit the chip): one kernel a checkpoint, so
   // a graph holds four checkpoints; past the end of a solve a kernel takes ~2 us
-  bool resident = bbpp_persist_ok(ctx, (int)sizeof(T));
+  bool resident = bbpp_persist_ok(ctx, (int)sizeof(T), replace_every);
   const int single_chunk = (replace_every % 2 == 0) ? replace_every : 2 * replace_every;
   const int resident_chunk = replace_every <= (1 << 28) ? 4 * replace_every : replace_every;
   int chunk = resident ? resident_chunk : single_chunk;

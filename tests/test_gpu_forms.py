@@ -79,3 +79,14 @@ def test_no_memory_for_a_form(bbpp_lib, monkeypatch, form, dims):
     assert L.bbpp_debug_wait(s.handle, 0, 0) == 0
     x, rep = s.solve_host(b, None, **kw)
     assert rep.status == bbpp.CONVERGED and not np.array_equal(x, x2)
+
+
+def test_a_checkpoint_every_iteration_goes_one_by_one(bbpp_lib, monkeypatch):
+    """Neither a pair nor a resident launch has more than one iteration to do then."""
+    s, mask, rhs = make(monkeypatch, "default")
+    x, _ = s.solve_host(rhs, mask, tol=1e-8, precision=bbpp.FP32_IR, replace_every=1)
+    s.set_profiling(True)
+    y, _ = s.solve_host(rhs, mask, tol=1e-8, precision=bbpp.FP32_IR, replace_every=1)
+    kinds = {k[0] for k in s.kernel_stats()}
+    assert "fused_f32" in kinds and not kinds & FORMS["default"]
+    assert np.array_equal(x, y)  # without profiling the same kernels

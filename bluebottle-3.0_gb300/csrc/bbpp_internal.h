@@ -220,6 +220,8 @@ int bbpp_pcg_loop_pair(bbpp_ctx *ctx, const uint8_t *mask, const float *rhs, flo
 // iterations up to the next checkpoint in one resident kernel (bbpp_persist.cu)
 void bbpp_persist_init(bbpp_ctx *ctx);
 void bbpp_persist_free(bbpp_ctx *ctx);
+size_t bbpp_persist_bytes(const bbpp_ctx *ctx);
+void bbpp_persist_attach(bbpp_ctx *ctx, void *p);
 bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem, int replace_every);
 bool bbpp_one_step(const bbpp_ctx *ctx);  // a one-iteration FP32 form was asked for
 int bbpp_persist_begin(bbpp_ctx *ctx);

@@ -43,6 +43,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "bbpp_internal.h"
@@ -771,12 +772,19 @@ void bbpp_pair_init(bbpp_ctx *ctx) {
   const size_t smem = ((size_t)RING * (ty + 4) + (size_t)(RING + 2) * (ty + 2) + (size_t)XRING * ty) * G.nx * 4;
   const size_t need = std::max(smem, sizeof(float) * NDOT * (size_t)threads);
   if (need > (size_t)kPairSmem) return;
-  for (int v = 0; v < 16; v++)
-    if (cudaFuncSetAttribute(pick_pair(v & 1, v & 2, v & 4, v & 8), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kPairSmem) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
+  // once per device: sixteen calls
+  static std::atomic<bool> capped[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !capped[dev].load()) {
+    for (int v = 0; v < 16; v++)
+      if (cudaFuncSetAttribute(pick_pair(v & 1, v & 2, v & 4, v & 8), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kPairSmem) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+      }
+    if (dev < 64) capped[dev].store(true);
+  }
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_pair(true, true, G.iso != 0, !(G.px && G.py)), threads,
                                                     need) != cudaSuccess ||

@@ -337,7 +337,11 @@ extern "C" int bbpp_create(const bbpp_grid *g, bbpp_ctx **out) {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
   ctx->stream = ctx->own_stream;
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->st, sizeof(DevState) * 2);
+  // two states and, on a line of its own, the exchange of the resident iteration
+  static_assert(sizeof(DevState) % 128 == 0, "lines");
+  const size_t st_bytes = sizeof(DevState) * 2 + bbpp_persist_bytes(ctx);
+  if (e == cudaSuccess) e = cudaMalloc(&ctx->st, st_bytes);
+  if (e == cudaSuccess) bbpp_persist_attach(ctx, ctx->st + 2);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->partials, sizeof(double) * 3 * nparts);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->r, sizeof(double) * n);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->p[0], sizeof(double) * n);
@@ -346,7 +350,7 @@ extern "C" int bbpp_create(const bbpp_grid *g, bbpp_ctx **out) {
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->hst, sizeof(DevState) * 2);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->st, 0, sizeof(DevState) * 2, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->st, 0, st_bytes, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->partials, 0, sizeof(double) * 3 * nparts, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {

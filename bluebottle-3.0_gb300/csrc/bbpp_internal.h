@@ -210,6 +210,7 @@ int bbpp_residual_async(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs, c
 void bbpp_pair_init(bbpp_ctx *ctx);
 void bbpp_pair_free(bbpp_ctx *ctx);
 bool bbpp_pair_ok(const bbpp_ctx *ctx);
+bool bbpp_pair_ready(const bbpp_ctx *ctx, bool mask);
 size_t bbpp_pair_partials(const bbpp_ctx *ctx);
 void bbpp_pair_launch(bbpp_ctx *ctx, bool step, const uint8_t *mask, const float *zin, const float *pin, float *zout,
                       float *pout, float *x, bbpp::DevState *st, int replace_every);
@@ -224,7 +225,7 @@ size_t bbpp_persist_bytes(const bbpp_ctx *ctx);
 void bbpp_persist_attach(bbpp_ctx *ctx, void *p);
 bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem, int replace_every);
 bool bbpp_one_step(const bbpp_ctx *ctx);  // a one-iteration FP32 form was asked for
-int bbpp_persist_begin(bbpp_ctx *ctx);
+bool bbpp_persist_begin(bbpp_ctx *ctx, int elem, bool mask);
 bool bbpp_persist_refused(bbpp_ctx *ctx, int elem, cudaError_t e);
 template <typename T>
 int bbpp_persist(bbpp_ctx *ctx, const uint8_t *mask, T *r, T *const p[2], T *Ap, T *x, bbpp::DevState *st,

@@ -3,7 +3,8 @@
 //
 // Restarted refinement: outer loop (FP64): r = rhs - (-A)x, stop when
 // ||r|| <= tol ||rhs||.
-// Inner sweep (FP32 vectors, FP64 dot accumulators across threads and CTAs):
+// Inner sweep (FP32 vectors, dot products summed across threads and CTAs no less
+// exactly than in FP64):
 // Jacobi PCG on (-A)d = r from d = 0 until ||r_d|| <= inner_tol ||r||, then
 // x += d in FP64.  The inner sweeps reuse the FP64 method's kernels
 // instantiated for float.
@@ -105,7 +106,7 @@ static int solve_reliable(bbpp_ctx *ctx, const uint8_t *mask, const double *rhs,
               (every ? !bbpp_tma_fused_ok(ctx) : !resident || n > 4200000);
   // a second z for the pairs, a second r and Ap for the fused iteration; without the memory the solve takes a
   // form that needs less
-  if (pair) pair = extra(ctx, &b->rd2);
+  if (pair) pair = extra(ctx, &b->rd2) && bbpp_pair_ready(ctx, mask != nullptr);
   if (pair) resident = false;
   bool fused = ctx->fused != 0 && bbpp_tma_fused_ok(ctx) && !resident && !pair;
   if (fused) fused = extra(ctx, &b->rd2) && extra(ctx, &b->Ap2);

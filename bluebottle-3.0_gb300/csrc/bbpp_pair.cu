@@ -754,6 +754,24 @@ PairKern pick_pair(bool step, bool mask, bool iso, bool wxy) {
   if (step) return mask ? pick2<true, true>(iso, wxy) : pick2<true, false>(iso, wxy);
   return mask ? pick2<false, true>(iso, wxy) : pick2<false, false>(iso, wxy);
 }
+
+// The kernel's shared memory cap, once per device and kernel; only the kernels that run
+// are loaded for it (all sixteen, when a context was made, took 9 ms of a process's first).
+bool pair_cap(const GeoL &G, bool step, bool mask) {
+  static std::atomic<unsigned int> capped[64];
+  const bool iso = G.iso != 0, wxy = !(G.px && G.py);
+  const unsigned int bit = 1u << (8 * (int)step + 4 * (int)mask + 2 * (int)iso + (int)wxy);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 64 && (capped[dev].load() & bit)) return true;
+  if (cudaFuncSetAttribute(pick_pair(step, mask, iso, wxy), cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (dev < 64) capped[dev].fetch_or(bit);
+  return true;
+}
 }  // namespace
 
 void bbpp_pair_init(bbpp_ctx *ctx) {
@@ -772,19 +790,7 @@ void bbpp_pair_init(bbpp_ctx *ctx) {
   const size_t smem = ((size_t)RING * (ty + 4) + (size_t)(RING + 2) * (ty + 2) + (size_t)XRING * ty) * G.nx * 4;
   const size_t need = std::max(smem, sizeof(float) * NDOT * (size_t)threads);
   if (need > (size_t)kPairSmem) return;
-  // once per device: sixteen calls
-  static std::atomic<bool> capped[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !capped[dev].load()) {
-    for (int v = 0; v < 16; v++)
-      if (cudaFuncSetAttribute(pick_pair(v & 1, v & 2, v & 4, v & 8), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kPairSmem) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-      }
-    if (dev < 64) capped[dev].store(true);
-  }
+  if (!pair_cap(G, true, true)) return;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_pair(true, true, G.iso != 0, !(G.px && G.py)), threads,
                                                     need) != cudaSuccess ||
@@ -806,6 +812,10 @@ void bbpp_pair_free(bbpp_ctx *ctx) {
 }
 
 bool bbpp_pair_ok(const bbpp_ctx *ctx) { return ctx->pair && ctx->pair->ok; }
+
+bool bbpp_pair_ready(const bbpp_ctx *ctx, bool mask) {
+  return pair_cap(ctx->GL, false, mask) && pair_cap(ctx->GL, true, mask);
+}
 
 // CTAs x products over the three sums of a CTA that the context sizes by
 size_t bbpp_pair_partials(const bbpp_ctx *ctx) {

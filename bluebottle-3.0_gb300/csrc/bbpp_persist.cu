@@ -213,8 +213,9 @@ __device__ __forceinline__ void exchange(const double (&v)[NV], double (&tot)[NV
 }
 
 // The same for the NV products of a one-exchange iteration (NV <= 7), each summed by a
-// warp of its own: over the CTA's threads (sum_floats), then over the CTAs' slots, in fixed order.  Warp 7 counts the CTA
-// in, its earlier global writes before it, and waits.  Totals in s_tot.
+// warp of its own: over the CTA's threads (sum_floats), then over the CTAs' slots, in
+// fixed order.  Warp 7 counts the CTA in, its earlier global writes before it, and
+// waits.  Totals in s_tot.
 template <int NV, int NTH>
 __device__ __forceinline__ void exchange_all(const float (&v)[NV], double *s_tot, bbpp_exchange *ex,
                                              Slot (*slots)[kMaxCtas], int nb, unsigned long long n,
@@ -1128,24 +1129,6 @@ void bbpp_persist_init(bbpp_ctx *ctx) {
       ok = plan_boxes(ctx->GL, most, elem, 512, false, &B);
       B.level = 0;
     }
-    const int all = kSmemCap - (int)static_smem(t->nth[k]);
-    if (!ok) continue;
-    // the attribute is a per-function cap shared by all contexts: the maximum,
-    // set once per device (setting it and asking for the occupancy take ~1 ms)
-    static std::atomic<unsigned int> ready[64];
-    const int variant = 8 * k + 4 * B.one + (t->nth[k] == 256 ? 3 : B.level);
-    const bool known = dev < 64 && (ready[dev].load() >> variant & 1u);
-    for (int v = 0; v < 4 && ok && !known; v++) {
-      const void *f = k ? (const void *)pick(0.0, t->nth[k], B, v & 1, v & 2)
-                        : (const void *)pick(0.f, t->nth[k], B, v & 1, v & 2);
-      ok = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, all) == cudaSuccess;
-      int per_sm = 0;
-      ok = ok &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, t->nth[k], (size_t)all) == cudaSuccess &&
-           per_sm >= 1;
-    }
-    cudaGetLastError();
-    if (ok && dev < 64) ready[dev].fetch_or(1u << variant);
     t->ok[k] = ok;
   }
 }
@@ -1174,17 +1157,36 @@ bool bbpp_persist_ok(const bbpp_ctx *ctx, int elem, int replace_every) {
   return ctx->persist && ctx->persist->ok[elem == 8 ? 1 : 0] && !ctx->profiling;
 }
 
-// Before a solve's first resident kernel: arrivals count from zero (a launch
-// whose wait ran out leaves them uneven).  Epochs run on.
-int bbpp_persist_begin(bbpp_ctx *ctx) {
-  bbpp_exchange *ex = ctx->persist->ex;
-  cudaError_t e = cudaMemsetAsync(&ex->base, 0, sizeof(ex->base), ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&ex->arrived, 0, sizeof(ex->arrived), ctx->stream);
-  if (e != cudaSuccess) {
-    bbpp_record_error(ctx, e, "bbpp_persist_begin", __LINE__);
-    return BBPP_CUDA_ERROR;
+// Before a solve's first resident kernel: its shared memory, and arrivals count from zero
+// (a launch whose wait ran out leaves them uneven; epochs run on).  False: no resident
+// kernel here.  The attribute is a per-function cap shared by all contexts, so it is the
+// maximum, set once per device; only the kernel that runs is loaded for it (all of a
+// context's, when it was made, took 5 ms of a process's first).
+bool bbpp_persist_begin(bbpp_ctx *ctx, int elem, bool mask) {
+  bbpp_persist_state *t = ctx->persist;
+  const int k = elem == 8 ? 1 : 0, nth = t->nth[k];
+  const Boxes &B = t->box[k];
+  const bool iso = ctx->GL.iso != 0;
+  static std::atomic<unsigned long long> ready[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit =
+      1ull << (32 * k + 16 * B.one + 4 * (nth == 256 ? 3 : B.level) + 2 * (int)mask + (int)iso);
+  if (dev >= 64 || !(ready[dev].load() & bit)) {
+    const void *f = k ? (const void *)pick(0.0, nth, B, mask, iso) : (const void *)pick(0.f, nth, B, mask, iso);
+    const int all = kSmemCap - (int)static_smem(nth);
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, all) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, nth, (size_t)all) != cudaSuccess || per_sm < 1) {
+      cudaGetLastError();
+      t->ok[k] = false;
+      return false;
+    }
+    if (dev < 64) ready[dev].fetch_or(bit);
   }
-  return 0;
+  cudaError_t e = cudaMemsetAsync(&t->ex->base, 0, sizeof(t->ex->base), ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(&t->ex->arrived, 0, sizeof(t->ex->arrived), ctx->stream);
+  return e == cudaSuccess;  // the solve's next call reports it
 }
 
 // Was the resident launch refused (the last bbpp_persist, or, with e, the launch of a graph of it)?  Then the

@@ -786,11 +786,11 @@ int bbpp_pcg_loop(bbpp_ctx *ctx, const uint8_t *mask, const T *rhs, T *x, T *r, 
                   DevState *hst, int replace_every, bool confirm, bool rr, int *iters_out) {
   // resident iterations (grids that fit the chip): one kernel a checkpoint, so
   // a graph holds four checkpoints; past the end of a solve a kernel takes ~2 us
-  bool resident = bbpp_persist_ok(ctx, (int)sizeof(T), replace_every);
+  bool resident =
+      bbpp_persist_ok(ctx, (int)sizeof(T), replace_every) && bbpp_persist_begin(ctx, (int)sizeof(T), mask != nullptr);
   const int single_chunk = (replace_every % 2 == 0) ? replace_every : 2 * replace_every;
   const int resident_chunk = replace_every <= (1 << 28) ? 4 * replace_every : replace_every;
   int chunk = resident ? resident_chunk : single_chunk;
-  if (resident && bbpp_persist_begin(ctx)) return BBPP_CUDA_ERROR;
   // a cooperative launch that is refused (fewer SMs than the device reports): the solve, at whose state nothing
   // has touched, and the context's later ones go on kernel by kernel
   auto refused = [&](cudaError_t e) {
@@ -1300,7 +1300,7 @@ __device__ __forceinline__ double mul_pow2(double v, double m, int k) {
 
 // PP_rhs (src/solver_kernel.cu:152-173) on dense face arrays: rhs = -(rho/dt)
 // div u*, the reference's evaluation order without contraction.  Bound by the FP64
-// pipe (9 instructions a cell); on spacings of 1 / 2^k, the usual ones, six
+// pipe (10 instructions a cell); on spacings of 1 / 2^k, the usual ones, seven
 // (POW2): at 256^3 333 us before, 244 now.
 template <bool POW2>
 __global__ void __launch_bounds__(256) k_rhs_div(const Geo G, double idx, double idy, double idz, int kx, int ky,

@@ -41,6 +41,7 @@ enum Inject : int {
   INJECT_REFUSED = 3,    // resident: the host takes the launch for refused
   INJECT_NO_MEMORY = 4,  // FP32: no memory for the vectors that only pairs and the fused iteration need
   INJECT_EXCHANGE = 5,   // resident, FP32 and FP64: the last CTA leaves the first exchange out
+  INJECT_DIRECTION = 6,  // pairs: every sixth takes its direction for lost
 };
 
 // Device-resident scalar state of one PCG solve.

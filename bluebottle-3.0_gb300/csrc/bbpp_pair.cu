@@ -125,12 +125,12 @@ __device__ __forceinline__ float4 fma4(const float2 a, const float4 b, const flo
 // What the end of a dots kernel reads of the state, at once: one load after another,
 // between the stores, would take an L2 latency each.
 struct PairIn {
-  int iter, stop, max_iter, fq, fresh, maxgap, last_rep;
+  int iter, stop, max_iter, fq, fresh, maxgap, last_rep, inject;
   double tol2bb, expected, rep_d2, rr_ref;
 };
 __device__ __forceinline__ PairIn pair_in(const DevState *st) {
   return {st->iter,     st->stop,    st->max_iter, st->fq,     st->pair_fresh, st->rep_maxgap,
-          st->last_rep, st->tol2bb,  st->rz_next,  st->rep_d2, st->rr_ref};
+          st->last_rep, st->inject,  st->tol2bb,  st->rz_next,  st->rep_d2, st->rr_ref};
 }
 
 // The end of a dots kernel: convergence of the residual at the pair's start,
@@ -155,7 +155,8 @@ __device__ static void pair_finish(DevState *st, const PairIn &in, const double 
     st->done = DONE_MAX_ITER;
     return;
   }
-  const PairPlan o = pair_plan(d, in.fresh == in.fq, in.expected);
+  const bool spoil = in.inject == INJECT_DIRECTION && in.fq % 6 == 5;
+  const PairPlan o = pair_plan(d, in.fresh == in.fq, spoil ? 0.0 : in.expected);
   const int n = ((it + 1) % replace_every == 0 || it + 1 > in.max_iter) ? 1 : o.steps;
   st->pAp = d[2];
   st->pair[0] = o.a0;

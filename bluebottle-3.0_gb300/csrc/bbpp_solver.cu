@@ -1348,7 +1348,7 @@ extern "C" int bbpp_rhs_div(bbpp_ctx *ctx, double rho_f, double dt, const double
 extern "C" int bbpp_debug_wait(bbpp_ctx *ctx, long long wait_ns, int inject) {
   if (!ctx || wait_ns < 0) return BBPP_BAD_ARG;
   ctx->wait_ns = wait_ns;
-  ctx->inject = inject >= INJECT_LAST_WAIT && inject <= INJECT_EXCHANGE ? inject : (inject ? INJECT_COPIES : 0);
+  ctx->inject = inject >= INJECT_LAST_WAIT && inject <= INJECT_DIRECTION ? inject : (inject ? INJECT_COPIES : 0);
   return 0;
 }
 

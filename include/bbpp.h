@@ -319,7 +319,8 @@ const char *bbpp_version(void);
  * (the resident iteration an exchange).  2: the last CTA of the resident iteration (FP32 and FP64) takes the
  * wait that ends a solve for run out.  3: the resident iteration's launch is taken for refused (the solve goes
  * on kernel by kernel, as do the context's later ones).  4: FP32 solves find no memory for the vectors that only
- * some forms of their iteration need (and take another).  5: as 1 for the resident iteration, FP64 too.  Nothing faults or hangs; the context stays usable. */
+ * some forms of their iteration need (and take another).  5: as 1 for the resident iteration, FP64 too.  6: every
+ * sixth pair of FP32 iterations takes its search direction for lost (and goes on along the residual).  Nothing faults or hangs; the context stays usable. */
 int bbpp_debug_wait(bbpp_ctx *ctx, long long wait_ns, int inject);
 /* Select the GPU for this host thread's later contexts and buffers (one process per GPU; no counterpart in
  * the reference, whose ranks each own one GPU through cudaSetDevice in its start-up code). */

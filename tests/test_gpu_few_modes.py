@@ -101,3 +101,27 @@ def test_isolated_fluid_cells(bbpp_lib, monkeypatch, form, bc):
     # FP32 leaves 6e-8 of the residual after one step, so a second and a confirmation's third
     assert rep.status == bbpp.CONVERGED and rep.iters <= 4
     assert np.linalg.norm(x - xe) <= 4 * 1e-8 * np.linalg.norm(xe)
+
+
+@pytest.mark.parametrize("dims,bc", [((64, 45, 30), "ppn"), ((48, 40, 33), "nnn"), ((256, 29, 20), "ppp")])
+def test_pairs_that_lose_their_direction(bbpp_lib, monkeypatch, dims, bc):
+    """Every sixth pair goes along z instead of p (a test hook): one step, and
+    conjugate gradients from there.  Each stretch reduces the error, so the solve
+    converges, if later than one that keeps its directions."""
+    monkeypatch.setenv("BBPP_PERSIST", "0")
+    nx, ny, nz = dims
+    g = bbpp.Grid.make(nx, ny, nz, 1.0 / nx, 1.0 / ny, 1.0 / nz, problems.bc_tuple(bc))
+    rng = np.random.default_rng(7)
+    mask = (rng.random(g.shape) < 0.05).astype(np.uint8)
+    b = rng.uniform(-1, 1, g.shape)
+    b[mask == 1] = 0
+    b[mask == 0] -= b[mask == 0].mean()
+    kw = dict(tol=1e-8, precision=bbpp.FP32_IR)
+    s = bbpp.Solver(g)
+    x0, rep0 = s.solve_host(b, mask, **kw)
+    assert bbpp.lib().bbpp_debug_wait(s.handle, 0, 6) == 0
+    x, rep = s.solve_host(b, mask, **kw)
+    assert rep.status == bbpp.CONVERGED and rep.true_rel <= 1.01e-8
+    assert rep.iters > rep0.iters
+    # both within tol of a zero residual, the condition number below (2 n / pi)^2
+    assert np.abs(x - x0).max() <= (2 * max(dims) / np.pi) ** 2 * 1e-8 * np.abs(x0).max()

@@ -142,13 +142,13 @@ __device__ static void pair_finish(DevState *st, const PairIn &in, const double 
   st->rz_last = rz;
   st->rr = rr;
   st->rz = rz;
-  st->rz_next = rz;
   if (isnan(rz)) {
     st->done = DONE_NAN;
     return;
   }
   if (it > 0 && (in.stop == 0 ? rz : rr) <= in.tol2bb) {
     st->done = it > in.max_iter ? DONE_MAX_ITER : (in.stop == 0 ? DONE_CONVERGED : DONE_PENDING);
+    st->rz_next = rz;  // what a confirmation compares with
     return;
   }
   if (it > in.max_iter) {
@@ -664,7 +664,14 @@ __global__ void __launch_bounds__(PNT, 1) k_pair(const GeoL G, const PairShape S
   double *sd = reinterpret_cast<double *>(smem_raw);
   for (int k = tid >> 5; k < NDOT; k += nth >> 5) {
     double a = 0.0;
-    for (unsigned int b = lane; b < nb; b += 32) a += __ldcg(&partials[(size_t)k * nb + b]);
+    for (unsigned int b0 = lane; b0 < nb; b0 += 256) {  // eight loads at once
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] = b0 + 32 * i < nb ? __ldcg(&partials[(size_t)k * nb + b0 + 32 * i]) : 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (b0 + 32 * i < nb) a += v[i];
+    }
     a = warp_sum(a);
     if (lane == 0) sd[k] = a;
   }
